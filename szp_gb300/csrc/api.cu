@@ -91,7 +91,6 @@ std::mutex g_mu;
 int g_segments = 0;
 int g_timing = 0;
 int g_overlap = -1;  // locate overlap override (tests of the repair paths)
-int g_decode_tickets = 0;  // single-field decode draws tickets (tests of that path)
 unsigned long long g_launches = 0;
 
 int resolve_segments(int requested) {
@@ -161,6 +160,14 @@ struct Workspace {
   int ev_pending[kNumSlots];  // recorded and not yet read
   int ev_last[kNumSlots];     // most recent completed pair
   int sm_count = 0;
+
+  // Look-back words; new ones are zeroed, so that none looks ready by chance.
+  cudaError_t ensure_status(size_t bytes, cudaStream_t st) {
+    const size_t had = status.cap;
+    cudaError_t e = status.ensure(bytes);
+    if (e == cudaSuccess && status.cap != had) e = cudaMemsetAsync(status.p, 0, status.cap, st);
+    return e;
+  }
 
   int init(int dev) {
     device = dev;
@@ -355,7 +362,7 @@ int compress_launch(Workspace& w, const CompressJob& j, cudaStream_t st) {
   tile_counts(sg, fm2, tb, per_seg, ntiles);
   if (ntiles >= (1ull << 31) || per_seg >= (1ull << 31))
     return fail(SZP_GB300_EINVAL, "input too large for one launch");
-  CU(w.status.ensure(ntiles * sizeof(uint64_t)));
+  CU(w.ensure_status(ntiles * sizeof(uint64_t), st));
   DevMisc* dm = w.dm();
   if (!j.keep_err) CU(cudaMemsetAsync(&dm->err, 0, sizeof(uint32_t), st));
 
@@ -479,28 +486,31 @@ int decompress_launch(Workspace& w, const DecompressJob& j, cudaStream_t st) {
   if (codes && !f64_pipe_supported((uint32_t)j.L))
     return fail(SZP_GB300_EINVAL, "code streams take blockSize 8..256 (got %d)", j.L);
   const bool fm2 = j.fm == 2;
-  const bool qpipe = codes || (dbl && f64_pipe_supported((uint32_t)j.L));  // a pipeline writing doubles or codes
+  const bool flow = flow_supported((uint32_t)j.L);  // decode_flow, else the per-block passes
   Segments sg = make_segments(j.n, j.T, j.L);
   const uint32_t maxsz = fm2 ? (j.L == 1 ? 5u : 4 + block_bytes((uint32_t)j.L - 1, kMaxBitCount))
                              : max_block_bytes((uint32_t)j.L);
   if (maxsz > 16384) return fail(SZP_GB300_EINVAL, "blockSize %d too large", j.L);
   const uint32_t C = locate_chunk_bytes(maxsz);
-  const uint32_t SC = locate_super_bytes(maxsz);
+  const uint32_t SC = flow ? flow_chunk_bytes((uint32_t)j.L) : locate_super_bytes(maxsz);
   const uint64_t nlocate = (j.len + SC - 1) / SC + (uint64_t)j.T + 1;
   uint32_t bpw = 1;
-  uint32_t tb = dbl && !qpipe ? decode_blocks_per_tile_f64((uint32_t)j.L, bpw)
-                              : decode_blocks_per_tile((uint32_t)j.L, bpw);
+  const uint32_t tb = decode_blocks_per_tile((uint32_t)j.L, bpw);
   uint64_t per_seg, ntiles;
   tile_counts(sg, fm2, tb, per_seg, ntiles);
   uint64_t nblk_total = 0;
   if (sg.n) {
     nblk_total = (uint64_t)(sg.T - 1) * (sg.tsz ? seg_blocks_host(sg, 0, fm2) : 0) + seg_blocks_host(sg, sg.T - 1, fm2);
   }
-  if (ntiles >= (1ull << 31) || nlocate >= (1ull << 31)) return fail(SZP_GB300_EINVAL, "input too large");
-  const uint64_t nstatus = ntiles > nlocate ? ntiles : nlocate;
-  CU(w.status.ensure(nstatus * sizeof(uint64_t)));
-  CU(w.walks.ensure(nlocate * sizeof(uint2)));
-  CU(w.blkpos.ensure((nblk_total + 1) * sizeof(uint32_t)));
+  if ((!flow && ntiles >= (1ull << 31)) || nlocate >= (1ull << 31)) return fail(SZP_GB300_EINVAL, "input too large");
+  if (flow) {
+    CU(w.ensure_status(2 * nlocate * sizeof(uint64_t), st));
+    CU(w.walks.ensure(nlocate * sizeof(uint4)));
+  } else {
+    CU(w.ensure_status(std::max(ntiles, nlocate) * sizeof(uint64_t), st));
+    CU(w.walks.ensure(nlocate * sizeof(uint2)));
+    CU(w.blkpos.ensure((nblk_total + 1) * sizeof(uint32_t)));
+  }
   const size_t plan_bytes = 64 + 4ull * (j.T + 1) + 16ull * j.T + 64;
   CU(w.plan.ensure(plan_bytes));
   DevMisc* dm = w.dm();
@@ -536,31 +546,32 @@ int decompress_launch(Workspace& w, const DecompressJob& j, cudaStream_t st) {
   f.yd = j.d_yd;
   f.ntiles = (uint32_t)ntiles;
   f.tiles_per_seg = (uint32_t)per_seg;
-  f.tile_base = 0;
-  f.loc_base = 0;
-  f.loc_ctas = (uint32_t)nlocate;
   a.ntiles = (uint32_t)ntiles;
   a.tb = tb;
   a.bpw = bpw;
   a.nlocate_ctas = (uint32_t)nlocate;
-  a.static_tiles = g_decode_tickets ? 0u : 1u;
-  if (((!dbl || qpipe) && decode_smem_bytes((uint32_t)j.L, tb, fm2) > 200 * 1024) ||
-      locate_smem_bytes(SC, a.overlap, maxsz) > 200 * 1024)
+  if (flow) {
+    a.out_kind = codes ? (j.accumulate ? kOutCodesAdd : kOutCodes) : dbl ? kOutDouble : kOutFloat;
+    f.y = static_cast<float*>(yout);
+    a.map = w.walks.as<uint4>();
+    a.ticket_total = &f.plan->nchunks;
+  } else if (locate_smem_bytes(SC, a.overlap, maxsz) > 200 * 1024) {
     return fail(SZP_GB300_EINVAL, "blockSize too large");
-  if (qpipe) f.y = reinterpret_cast<float*>(codes ? (void*)j.d_codes : (void*)j.d_yd);  // it writes doubles or codes
+  }
   CU(cudaMemsetAsync(dm->verify, 0, sizeof(uint32_t), st));
 
   w.mark(kSlotSetup, 0, st);
   CU(launch_dec_setup(a, st));
   w.mark(kSlotSetup, 1, st);
-  w.mark(kSlotLocate, 0, st);
-  CU(launch_locate(a, st));
-  w.mark(kSlotLocate, 1, st);
+  if (!flow) {
+    w.mark(kSlotLocate, 0, st);
+    CU(launch_locate(a, st));
+    w.mark(kSlotLocate, 1, st);
+  }
   w.mark(kSlotDecode, 0, st);
-  CU(codes ? launch_decode_codes(a, j.accumulate, st)
-            : qpipe ? launch_decode_q(a, st) : dbl ? launch_decode_f64(a, st) : launch_decode(a, st));
+  CU(flow ? launch_decode_flow(a, st) : dbl ? launch_decode_f64(a, st) : launch_decode(a, st));
   w.mark(kSlotDecode, 1, st);
-  count_launches(3);
+  count_launches(flow ? 2 : 3);
   return SZP_GB300_OK;
 }
 
@@ -1508,7 +1519,7 @@ int szp_gb300_wait_probe(unsigned long long limit_ns, unsigned long long* waited
 void szp_gb300_set_timing(int enable) { g_timing = enable ? 1 : 0; }
 
 void szp_gb300_set_locate_overlap(int bytes) { g_overlap = bytes; }
-void szp_gb300_set_decode_tickets(int on) { g_decode_tickets = on ? 1 : 0; }
+void szp_gb300_set_decode_tickets(int) {}  // every decode draws tickets
 
 double szp_gb300_kernel_ms(int slot) {
   Workspace* w;

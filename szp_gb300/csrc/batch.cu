@@ -10,7 +10,7 @@
 //
 // Stages per run:
 //   compress    clear errors | range pass (REL fields) | compress tiles
-//   decompress  clear errors | header setup (one CTA per field) | locate | decode
+//   decompress  clear errors | header setup (one CTA per field) | decode
 //
 // The tile size (8*rounds*8 blocks of 32, rounds 1/2/4) is chosen per batch by
 // timing each candidate on the batch itself (SZP_GB300_BATCH_AUTOTUNE).
@@ -152,26 +152,19 @@ int build_compress(szp_gb300_batch_s& b, Config& c) {
 }
 
 int build_decompress(szp_gb300_batch_s& b, Config& c) {
-  const uint32_t tb = batch_tile_blocks(c.rounds);
   DecompressPlan p;
-  int rc = plan_decompress(b.fields.data(), b.nfields, b.L, b.T, tb, p);
+  int rc = plan_decompress(b.fields.data(), b.nfields, b.L, b.T, p);
   if (rc) return rc;
-  if (p.tiles > b.status_words || p.locs > b.status_words)
+  if (2 * p.locs > b.status_words)
     return host_fail(SZP_GB300_EINVAL, "look-back words too few for the batch");
   uint8_t* d_plans;
-  uint32_t* d_blkpos;
-  uint2* d_aux;
+  uint4* d_map;
   BCU(c.al.get(&d_plans, p.plan_stride * (size_t)b.nfields + 16));
-  BCU(c.al.get(&d_blkpos, p.blocks + 1));
-  BCU(c.al.get(&d_aux, p.locs + 1));
-  place_decompress(p, d_plans, d_blkpos, b.d_err);
+  BCU(c.al.get(&d_map, p.locs + 1));
+  place_decompress(p, d_plans, b.d_err);
   DecField* d_fields;
-  uint32_t *d_tile_field, *d_loc_field;
   BCU(upload(c.al, &d_fields, p.fields));
-  BCU(upload(c.al, &d_tile_field, p.tile_field));
-  BCU(upload(c.al, &d_loc_field, p.loc_field));
-  args_decompress(c.da, p, d_fields, d_tile_field, d_loc_field, d_aux, b.d_misc->counters, b.d_status,
-                  &b.d_misc->ls, &b.d_misc->err, tb);
+  args_decompress(c.da, p, d_fields, d_map, b.d_misc->counters, b.d_status, &b.d_misc->ls, &b.d_misc->err);
   c.nfields = (uint32_t)b.nfields;
   return SZP_GB300_OK;
 }
@@ -181,7 +174,7 @@ int issue(szp_gb300_batch_s& b, const Config& c, cudaStream_t st) {
   BCU(cudaMemsetAsync(b.d_err, 0, sizeof(uint32_t) * (size_t)b.nfields, st));
   BCU(cudaMemsetAsync(&b.d_misc->err, 0, sizeof(uint32_t) * 5, st));  // launch error + counters
   if (b.dir == SZP_GB300_BATCH_COMPRESS) return issue_compress(c.ca, c.ra, c.rel_grid, c.rounds, st);
-  return issue_decompress(c.da, c.nfields, c.rounds, st);
+  return issue_decompress(c.da, c.nfields, st);
 }
 
 int make_config(szp_gb300_batch_s& b, int rounds, Config** out) {
@@ -300,13 +293,10 @@ void place_compress(CompressPlan& p, unsigned long long* d_sizes, uint32_t* d_er
   }
 }
 
-int plan_decompress(const szp_gb300_field* fl, int nf, int L, int T, uint32_t tb, DecompressPlan& p) {
-  const uint32_t maxsz = max_block_bytes((uint32_t)L);
-  const uint32_t SC = locate_super_bytes(maxsz);
+int plan_decompress(const szp_gb300_field* fl, int nf, int L, int T, DecompressPlan& p) {
+  const uint32_t SC = flow_chunk_bytes((uint32_t)L);
   p.fields.assign(nf, DecField{});
-  p.tile_field.clear();
-  p.loc_field.clear();
-  p.tiles = p.locs = p.blocks = 0;
+  p.locs = 0;
   p.plan_stride = ((sizeof(DecPlan) + 16ull * T + 4ull * (T + 1)) + 15) & ~(size_t)15;
   for (int f = 0; f < nf; f++) {
     const szp_gb300_field& in = fl[f];
@@ -320,29 +310,15 @@ int plan_decompress(const szp_gb300_field* fl, int nf, int L, int T, uint32_t tb
     df.seg.L = (uint32_t)L;
     df.seg.tsz = in.nbEle / (uint64_t)T;
     df.plan = reinterpret_cast<DecPlan*>((uintptr_t)(p.plan_stride * (size_t)f));
-    df.nblk_total = host_block_count(in.nbEle, T, L);
-    df.blkpos = reinterpret_cast<uint32_t*>((uintptr_t)p.blocks);
     df.err = reinterpret_cast<uint32_t*>((uintptr_t)f);
     df.y = static_cast<float*>(in.output);
-    uint64_t per_seg = 0, nt = 0;
-    host_tile_counts(in.nbEle, T, L, tb, per_seg, nt);
-    df.ntiles = (uint32_t)nt;
-    df.tiles_per_seg = (uint32_t)per_seg;
-    df.tile_base = (uint32_t)p.tiles;
-    const uint64_t nloc = in.input_bytes / SC + (uint64_t)T + 1;
-    df.loc_base = (uint32_t)p.locs;
-    df.loc_ctas = (uint32_t)nloc;
-    p.tile_field.insert(p.tile_field.end(), nt, (uint32_t)f);
-    p.loc_field.insert(p.loc_field.end(), nloc, (uint32_t)f);
-    p.tiles += nt;
-    p.locs += nloc;
-    p.blocks += df.nblk_total;
-    if (p.tiles >= (1ull << 31) || p.locs >= (1ull << 31)) return host_fail(SZP_GB300_EINVAL, "batch too large");
+    p.locs += in.input_bytes / SC + (uint64_t)T + 1;
+    if (p.locs >= (1ull << 30)) return host_fail(SZP_GB300_EINVAL, "batch too large");
   }
   return SZP_GB300_OK;
 }
 
-void place_decompress(DecompressPlan& p, uint8_t* d_plans, uint32_t* d_blkpos, uint32_t* d_err) {
+void place_decompress(DecompressPlan& p, uint8_t* d_plans, uint32_t* d_err) {
   const int T = p.fields.empty() ? 1 : (int)p.fields[0].seg.T;
   for (auto& df : p.fields) {
     uint8_t* pb = d_plans + reinterpret_cast<uintptr_t>(df.plan);
@@ -350,7 +326,6 @@ void place_decompress(DecompressPlan& p, uint8_t* d_plans, uint32_t* d_blkpos, u
     df.reg0 = reinterpret_cast<uint64_t*>(pb + sizeof(DecPlan));
     df.reg1 = df.reg0 + T;
     df.chunk_base = reinterpret_cast<uint32_t*>(df.reg1 + T);
-    df.blkpos = d_blkpos + reinterpret_cast<uintptr_t>(df.blkpos);
     df.err = d_err + reinterpret_cast<uintptr_t>(df.err);
   }
 }
@@ -376,28 +351,23 @@ void args_compress(CompressArgs& a, RelBatchArgs& r, const CompressPlan& p, Comp
   r.chunk = kRelChunk;
 }
 
-void args_decompress(DecArgs& a, const DecompressPlan& p, const DecField* d_fields, const uint32_t* d_tile_field,
-                     const uint32_t* d_loc_field, uint2* aux, uint32_t* counters, uint64_t* status, LaunchState* ls,
-                     uint32_t* err, uint32_t tb) {
+void args_decompress(DecArgs& a, const DecompressPlan& p, const DecField* d_fields, uint4* map, uint32_t* counters,
+                     uint64_t* status, LaunchState* ls, uint32_t* err) {
   const uint32_t maxsz = max_block_bytes(kBatchL);
   memset(&a, 0, sizeof a);
   a.fm2 = false;
-  a.chunk = locate_chunk_bytes(maxsz);
-  a.super_chunk = locate_super_bytes(maxsz);
+  a.super_chunk = flow_chunk_bytes(kBatchL);
   a.overlap = locate_overlap_bytes(maxsz);
   a.maxsz = maxsz;
-  a.aux = aux;
   a.counters = counters;
   a.status = status;
   a.ls = ls;
   a.err = err;
-  a.ntiles = (uint32_t)p.tiles;
-  a.tb = tb;
-  a.bpw = tb / 8;
   a.nlocate_ctas = (uint32_t)p.locs;
+  a.out_kind = kOutFloat;
+  a.map = map;
+  a.ticket_total = counters + 1;  // cleared with the counters before every run
   a.fields = d_fields;
-  a.tile_field = d_tile_field;
-  a.loc_field = d_loc_field;
 }
 
 int issue_compress(const CompressArgs& a, const RelBatchArgs& r, uint32_t rel_grid, int rounds, cudaStream_t st) {
@@ -406,10 +376,9 @@ int issue_compress(const CompressArgs& a, const RelBatchArgs& r, uint32_t rel_gr
   return SZP_GB300_OK;
 }
 
-int issue_decompress(const DecArgs& a, uint32_t nfields, int rounds, cudaStream_t st) {
+int issue_decompress(const DecArgs& a, uint32_t nfields, cudaStream_t st) {
   BCU(launch_dec_setup_batch(a, nfields, st));
-  BCU(launch_locate_batch(a, st));
-  if (a.ntiles) BCU(launch_decode_batch(a, kBatchL, rounds, st));
+  if (nfields) BCU(launch_decode_flow_batch(a, st));
   return SZP_GB300_OK;
 }
 
@@ -455,9 +424,8 @@ int szp_gb300_batch_create(szp_gb300_batch* out, int direction, const szp_gb300_
     cudaError_t pe = direction == SZP_GB300_BATCH_COMPRESS ? prepare_compress_batch() : prepare_decompress_batch();
     if (pe != cudaSuccess) return fail_out(host_fail(SZP_GB300_ECUDA, cudaGetErrorString(pe)));
   }
-  // look-back words: the most tiles / locate tickets any tile size needs
-  const uint32_t maxsz = max_block_bytes((uint32_t)blockSize);
-  const uint32_t SC = locate_super_bytes(maxsz);
+  // look-back words: the most tiles any tile size needs (compression), two per super-chunk (decompression)
+  const uint32_t SC = flow_chunk_bytes((uint32_t)blockSize);
   uint64_t words = 1;
   {
     uint64_t tiles = 0, locs = 0;
@@ -465,7 +433,7 @@ int szp_gb300_batch_create(szp_gb300_batch* out, int direction, const szp_gb300_
       uint64_t ps, nt;
       host_tile_counts(fields[f].nbEle, T, blockSize, 64, ps, nt);  // the smallest tile (rounds 1)
       tiles += nt;
-      if (direction == SZP_GB300_BATCH_DECOMPRESS) locs += fields[f].input_bytes / SC + (uint64_t)T + 1;
+      if (direction == SZP_GB300_BATCH_DECOMPRESS) locs += 2 * (fields[f].input_bytes / SC + (uint64_t)T + 1);
     }
     words = std::max<uint64_t>(words, std::max(tiles, locs));
   }
@@ -487,9 +455,11 @@ int szp_gb300_batch_create(szp_gb300_batch* out, int direction, const szp_gb300_
   const int forced = (flags >> 8) & 0xF;
   if (forced && forced != 1 && forced != 2 && forced != 4)
     return fail_out(host_fail(SZP_GB300_EINVAL, "tile rounds must be 1, 2 or 4"));
+  // (decompression has no tiles to choose)
   std::vector<int> cand = forced ? std::vector<int>{forced}
-                         : (flags & SZP_GB300_BATCH_AUTOTUNE) ? std::vector<int>{4, 2, 1}
-                                                             : std::vector<int>{4};
+                         : direction == SZP_GB300_BATCH_COMPRESS && (flags & SZP_GB300_BATCH_AUTOTUNE)
+                             ? std::vector<int>{4, 2, 1}
+                             : std::vector<int>{4};
   float best = 0.0f;
   for (int r : cand) {
     Config* c = nullptr;
@@ -522,7 +492,7 @@ int szp_gb300_batch_run(szp_gb300_batch b, void* stream) {
     if (rc) return rc;
   }
   BCU(cudaEventRecord(b->done, st));
-  host_count_launches(b->dir == SZP_GB300_BATCH_COMPRESS ? (b->cfg->ra.nitems ? 2 : 1) : 3);
+  host_count_launches(b->dir == SZP_GB300_BATCH_COMPRESS ? (b->cfg->ra.nitems ? 2 : 1) : 2);
   return SZP_GB300_OK;
 }
 

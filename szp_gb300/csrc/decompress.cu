@@ -21,17 +21,12 @@
 //                 (entry, exit) pairs the predecessors published; a CTA whose
 //                 entry proves wrong re-walks from the true one.  Each chunk then
 //                 writes the header offset of each of its blocks.
-//  3. decode      decode_pipe (blockSize 8..256, a power of two), a persistent,
-//                 warp-specialised pipeline: per tile of blocks the stream span
-//                 and block offsets are staged in shared memory by TMA; LPB
-//                 lanes per block unpack 8 elements each (sign byte, byte
-//                 planes and remainder bits are byte-aligned per 8 elements),
-//                 prefix-add (fastmode1: warp and tile scans and a look-back
-//                 over the tiles of a segment; fastmode2: a scan inside the
-//                 block from its seed) and dequantize.  decode_generic covers
-//                 the other blockSizes.
-#include <atomic>
-
+//  3. decode      decode_generic: one warp per block, a look-back over the tiles
+//                 of a segment for the running q (fastmode1), or each block from
+//                 its seed (fastmode2).
+//
+// These are the passes of blockSizes other than 8, 16, ... 256, which
+// decode_flow (decode_flow.cu) takes in one kernel after dec_setup.
 #include <type_traits>
 
 #include "szp_device.cuh"
@@ -39,6 +34,7 @@
 #include "szp_kernels.h"
 #include "szp_pipe.cuh"
 #include "szp_tma.cuh"
+#include "szp_unpack.cuh"
 
 namespace szp {
 
@@ -52,10 +48,6 @@ __host__ __device__ __forceinline__ uint32_t full_block_size(uint32_t b, uint32_
   if (!fm2) return block_bytes(L, b);
   if (L == 1) return b == 0 ? 5u : 0u;
   return 4 + block_bytes(L - 1, b);
-}
-
-__host__ __device__ __forceinline__ uint32_t max_walk_block(uint32_t L, bool fm2) {
-  return fm2 ? (L == 1 ? 5u : 4 + block_bytes(L - 1, kMaxBitCount)) : block_bytes(L, kMaxBitCount);
 }
 
 constexpr int kLocThreads = 128;
@@ -84,6 +76,36 @@ __device__ __forceinline__ uint64_t load_u64le(const uint8_t* p) {
 // ---------------------------------------------------------------------------
 // 1. header -> plan
 // ---------------------------------------------------------------------------
+// Element e of the field's output from its code, in the launch's output kind.
+__device__ void put_seed(const DecArgs& a, const DecField& fd, uint64_t e, uint32_t q, float eb, double ebd) {
+  if (a.out_kind == kOutDouble) {
+    reinterpret_cast<unsigned long long*>(fd.y)[e] = DequantD(ebd)(q);
+  } else if (a.out_kind == kOutCodes) {
+    reinterpret_cast<uint32_t*>(fd.y)[e] = q;
+  } else if (a.out_kind == kOutCodesAdd) {
+    int32_t* p = reinterpret_cast<int32_t*>(fd.y) + e;
+    const int32_t x = *p, z = (int32_t)((uint32_t)x + q);
+    *p = z;
+    if (((x ^ z) & ((int32_t)q ^ z)) < 0) atomicOr(fd.err, kErrQuantRange);
+  } else {
+    fd.y[e] = dequant(q, eb, !isfinite(eb));
+  }
+}
+
+// Chunks in each super-chunk of a segment of nblk blocks in `bytes` bytes: as
+// many as hold 32 Ki values (empty blocks take one byte for 32 values, and a
+// CTA that meets thousands of them is the last to finish: a 2^24-value walk at
+// REL 1e-2 decodes 16 KB into 2 MB), and in a short stream no more than gives
+// the GPU two super-chunks per resident CTA (1 MB of floats: 22 -> 14 us).
+__device__ __forceinline__ uint32_t flow_chunks(const DecArgs& a, uint64_t bytes, uint64_t nblk, uint32_t L,
+                                                uint64_t total) {
+  // in single precision: the result only has to be the same wherever it is taken
+  const float most = (float)(kFlowSuper / a.super_chunk), c = (float)a.super_chunk;
+  const float by_values = __fdiv_rn((float)bytes * (32768.0f / L), fmaxf((float)nblk, 1.0f) * c);
+  const float by_total = __fdiv_rn((float)total, 2048.0f * c);
+  return (uint32_t)fmaxf(1.0f, fminf(most, fminf(by_values, by_total)));
+}
+
 template <bool BATCH>
 __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   const DecField& fd = BATCH ? a.fields[blockIdx.x] : a.f;
@@ -91,32 +113,40 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   const uint32_t T = sg.T;
   const uint32_t hb = a.hb == 8 ? 8u : 4u;  // eb header: float, or double (szpd_double.cc)
   const uint64_t head = hb + 8ull * T;
-  __shared__ uint32_t s_bad;
+  constexpr uint32_t kTurnT = 512;  // segments at most for the turns below
+  __shared__ uint32_t s_cb[kTurnT + 1], s_k[kTurnT];  // tickets before each segment; its chunks per super-chunk
+  __shared__ uint32_t s_bad, s_base0, s_all, s_most;  // s_most: of the segment with the most super-chunks
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   uint64_t len = fd.len;
   if (fd.len_dev) {
     uint64_t l2 = *fd.len_dev;
     len = l2 < len ? l2 : len;
   }
-  if (threadIdx.x == 0) {
-    s_bad = len < head ? 1u : 0u;
-    if (!s_bad) {
-      uint32_t b = ((uint32_t)fd.in[0] << 24) | ((uint32_t)fd.in[1] << 16) | ((uint32_t)fd.in[2] << 8) | fd.in[3];
-      fd.plan->eb = __uint_as_float(b);
+  const bool hdr_ok = len >= head;
+  if (threadIdx.x == 0) s_bad = hdr_ok ? 0u : 1u;
+  float eb = 0.0f;
+  double ebd = 0.0;
+  if (hdr_ok && (threadIdx.x == 0 || (T > sg.n && sg.tsz <= 1) || sg.tsz == 1)) {  // every thread that may write a seed
+    eb = __uint_as_float((uint32_t)fd.in[0] << 24 | (uint32_t)fd.in[1] << 16 | (uint32_t)fd.in[2] << 8 | fd.in[3]);
+    if (hb == 8) {
       unsigned long long d = 0;
-      if (hb == 8)
-        for (int i = 0; i < 8; i++) d = (d << 8) | fd.in[i];
-      fd.plan->ebd = __longlong_as_double((long long)d);
-    } else {
-      fd.plan->eb = 0.0f;
-      fd.plan->ebd = 0.0;
+      for (int i = 0; i < 8; i++) d = (d << 8) | fd.in[i];
+      ebd = __longlong_as_double((long long)d);
     }
   }
+  if (threadIdx.x == 0) {
+    fd.plan->eb = eb;
+    fd.plan->ebd = ebd;
+  }
+  // chunks per super-chunk, in its place in a ticket
+  auto chunks = [&](uint64_t bytes, uint64_t nblk) -> uint32_t {
+    return flow_chunks(a, bytes, nblk, sg.L, gridDim.x * len) << kFlowFieldBits;
+  };
   __syncthreads();
-  const bool hdr_ok = !s_bad;
   for (uint32_t t = threadIdx.x; t < T; t += blockDim.x) {
     uint64_t len_t = sg.len(t);
     uint64_t r0 = 0, r1 = 0;
-    uint32_t nch = 0;
+    uint32_t nch = 0, k = 0;
     bool bad = false;
     if (len_t > 0 && hdr_ok) {
       uint64_t off = load_u64le(fd.in + hb + 8ull * t);
@@ -142,8 +172,18 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
             uint64_t bound = r0 + nblk * (uint64_t)a.maxsz;
             r1 = end < bound ? end : bound;
             if (nblk > 0 && r1 <= r0) bad = true;
+            if (!a.fm2 && a.map && len_t == 1) {  // a lone seed has no blocks: its value is written here
+              const uint8_t* sp = fd.in + start;
+              const uint32_t q = (uint32_t)sp[0] | (uint32_t)sp[1] << 8 | (uint32_t)sp[2] << 16 | (uint32_t)sp[3] << 24;
+              put_seed(a, fd, sg.lo(t), q, eb, ebd);
+            }
             if (r1 - r0 >= (1ull << 32)) bad = true;  // block offsets are 32-bit
-            nch = (uint32_t)((r1 - r0 + a.super_chunk - 1) / a.super_chunk);
+            uint32_t sc = a.super_chunk;
+            if (a.map) {
+              k = chunks(r1 - r0, nblk);
+              sc *= k >> kFlowFieldBits;
+            }
+            nch = (uint32_t)((r1 - r0 + sc - 1) / sc);
           }
         }
       }
@@ -154,23 +194,73 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
     }
     fd.reg0[t] = r0;
     fd.reg1[t] = r1;
-    fd.chunk_base[t + 1] = nch;
+    if (t < kTurnT) {
+      s_cb[t + 1] = nch;
+      s_k[t] = k;
+    } else {
+      fd.chunk_base[t + 1] = nch;
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t acc = 0;
-    fd.chunk_base[0] = 0;
-    if (s_bad) {
-      for (uint32_t t = 0; t < T; t++) fd.chunk_base[t + 1] = 0;
-      atomicOr(fd.err, kErrCorrupt);
-    } else {
-      for (uint32_t t = 0; t < T; t++) {
-        acc += fd.chunk_base[t + 1];
-        fd.chunk_base[t + 1] = acc;
-      }
+  if (warp == 0) {  // chunk counts -> the chunks before each segment
+    uint32_t acc = 0, most = 0;
+    if (lane == 0) fd.chunk_base[0] = s_cb[0] = 0;
+    for (uint32_t t0 = 0; t0 < T; t0 += 32) {
+      const uint32_t t = t0 + lane;
+      const uint32_t n = t >= T || s_bad ? 0u : t < kTurnT ? s_cb[t + 1] : fd.chunk_base[t + 1];
+      const uint32_t incl = acc + warp_incl_scan(n, lane);
+      most = max(most, __reduce_max_sync(0xffffffffu, n));
+      if (t < T) fd.chunk_base[t + 1] = incl;
+      if (t < T && t < kTurnT) s_cb[t + 1] = incl;
+      acc = __shfl_sync(0xffffffffu, incl, 31);
     }
-    fd.plan->nchunks = s_bad ? 0 : acc;
-    fd.plan->bad = s_bad;
+    if (lane == 0) {
+      if (s_bad) atomicOr(fd.err, kErrCorrupt);
+      fd.plan->nchunks = acc;
+      fd.plan->bad = s_bad;
+      s_all = acc;
+      s_most = most;
+      s_base0 = BATCH ? atomicAdd(a.ticket_total, acc) : 0u;  // the field's first ticket
+    }
+  }
+  if (!a.map) return;
+  __syncthreads();
+  const uint32_t all = s_all;
+  if (all == 0) return;
+  // The tickets of decode_flow: field, segment, position in it, look-back
+  // record (the records of a segment follow one another).  The segments take
+  // turns (first super-chunk of each, second of each, ...), so that the CTAs in
+  // flight stand near the fronts of all of them and a look-back has 1/T of
+  // them before it (a 512^3 field at T = 16: 0.373 -> 0.291 ms); what a segment
+  // has beyond 5/4 of the average comes last.
+  const uint32_t turns = T < 4 || T > kTurnT ? 0u : min(all, (all + all / 4 + T - 1) / T);
+  for (uint32_t j = warp; j < turns; j += nwarps) {
+    uint32_t at = s_base0;  // and the tickets of the turns before j
+    for (uint32_t t = lane; t < ((T + 31) & ~31u); t += 32)
+      at += __reduce_add_sync(0xffffffffu, t < T ? min(s_cb[t + 1] - s_cb[t], j) : 0u);
+    for (uint32_t t = lane; t < ((T + 31) & ~31u); t += 32) {
+      const uint32_t c0 = s_cb[min(t, T)], n = t < T ? s_cb[t + 1] - c0 : 0u;
+      const uint32_t has = __ballot_sync(0xffffffffu, n > j);
+      if (n > j)
+        a.map[at + __popc(has & ((1u << lane) - 1u))] = make_uint4(s_k[t] | blockIdx.x, t, j, s_base0 + c0 + j);
+      at += __popc(has);
+    }
+  }
+  // the rest, segment by segment; they come after the tickets of the turns
+  if (s_most <= turns) return;
+  uint32_t at = s_base0;
+  for (uint32_t t = 0; turns && t < T; t++) at += min(s_cb[t + 1] - s_cb[t], turns);
+  for (uint32_t t = 0; t < T; t++) {
+    const uint32_t c0 = t < kTurnT ? s_cb[t] : fd.chunk_base[t];
+    const uint32_t n = (t < kTurnT ? s_cb[t + 1] : fd.chunk_base[t + 1]) - c0;
+    if (n > turns) {
+      const uint64_t len_t = sg.len(t);
+      const uint32_t k = t < kTurnT ? s_k[t]
+                                    : chunks(fd.reg1[t] - fd.reg0[t], a.fm2 ? (len_t + sg.L - 1) / sg.L : sg.blocks_fm1(t));
+      for (uint32_t j = turns + threadIdx.x; j < n; j += blockDim.x)
+        a.map[at + (j - turns)] = make_uint4(k | blockIdx.x, t, j, s_base0 + c0 + j);
+    }
+    at += n > turns ? n - turns : 0u;
   }
 }
 
@@ -275,7 +365,7 @@ static bool locate_packs(uint32_t super_chunk, uint32_t maxsz) {
   return maxsz <= 254 && (uint64_t)super_chunk + maxsz < kRelEnd;
 }
 
-template <bool FM2, bool BATCH, bool PACK>
+template <bool FM2, bool PACK>
 __global__ void __launch_bounds__(kLocThreads) locate_kernel(const __grid_constant__ DecArgs a) {
   constexpr int NT = kLocThreads;
   extern __shared__ __align__(16) uint8_t s_bytes[];
@@ -286,15 +376,14 @@ __global__ void __launch_bounds__(kLocThreads) locate_kernel(const __grid_consta
   __shared__ __align__(8) uint64_t s_bar;
   uint32_t tile, epoch;
   draw_ticket(a.ls, a.nlocate_ctas, tile, epoch, s_tk);
-  // status and aux words are indexed by launch ticket, chunks by field-local ticket
-  const DecField& fd = BATCH ? a.fields[a.loc_field[tile]] : a.f;
-  const uint32_t lt = tile - fd.loc_base;
+  const DecField& fd = a.f;
+  const uint32_t lt = tile;
   const uint32_t nct = fd.plan->bad ? 0 : fd.chunk_base[fd.seg.T];
   if (lt >= nct) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const Segments sg = fd.seg;
   const uint32_t t = chunk_segment(fd.chunk_base, sg.T, lt);
-  const uint32_t first = fd.loc_base + fd.chunk_base[t];  // launch ticket of the segment's first chunk
+  const uint32_t first = fd.chunk_base[t];  // ticket of the segment's first chunk
   const uint32_t j = tile - first;
   const uint64_t R0 = fd.reg0[t];
   const uint32_t rlen = (uint32_t)(fd.reg1[t] - R0);
@@ -637,30 +726,6 @@ __device__ __forceinline__ uint32_t decode_delta(const uint8_t* __restrict__ hdr
   return neg ? 0u - v : v;
 }
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  return x;
-}
-
-// (float)q * eb (szpd_float.cc:67,86,112).  NaN can only appear when eb is
-// not finite; `special` (warp-uniform) selects the x86 NaN rule then.
-__device__ __forceinline__ float dequant(uint32_t q, float eb, bool special = false) {
-  float f = __int2float_rn((int32_t)q);
-  float r = __fmul_rn(f, eb);
-  return special ? x86_nan_fix(r, f, eb) : r;
-}
-
-// (double)q * eb for float64 streams (szpd_double.cc:67,86,112).
-__device__ __forceinline__ double dequant(uint32_t q, double eb, bool special = false) {
-  const double f = (double)(int32_t)q;
-  const double r = __dmul_rn(f, eb);
-  return special ? x86_nan_fix_d(r, f, eb) : r;
-}
-
 template <int WARPS>
 __device__ __forceinline__ uint32_t scan_warps_u32(uint32_t* s_w, uint32_t mine, int warp, int lane,
                                                    uint32_t& excl) {
@@ -709,723 +774,6 @@ __device__ __forceinline__ DecTile dec_tile(const Segments& sg, uint32_t tile, u
 
 
 constexpr int kDecWarps = 8;
-constexpr int kDecRounds = 4;
-
-// ---------------------------------------------------------------------------
-// fastmode1 decode, blockSize L = 8*LPB, as a persistent, warp-specialised
-// pipeline (the mirror of the compressor's):
-//   producer  draws tile tickets; stages the tile's block offsets and its
-//             stream span in a slot by bulk copy
-//   compute   unpacks the deltas (LPB lanes per block, 8 elements per lane:
-//             the byte layout of 8 elements is self-contained), scans them
-//             inside the tile and stages the tile-relative prefix sums (int32)
-//             in the slot, over the span they came from; then finishes the
-//             previous tile: adds its base, dequantizes, 16-byte stores
-//   control   looks back for each tile's base (the segment's seed plus the
-//             deltas of the tiles before it, szpd_float.cc:76-118) while the
-//             compute warps unpack the next tile
-// ---------------------------------------------------------------------------
-constexpr int kDecControl = 2;
-// Slots of a decode pipeline with ROUNDS rounds per warp: a tile is finished
-// (dequantized and stored) NS - 2 tiles after it was staged, so that its
-// base (the look-back over the tiles before it) has that long to arrive.
-// Tiles of 2 rounds (half the shared memory of 4) get 6 slots, 4 tiles of slack.
-template <int ROUNDS>
-__host__ __device__ constexpr int dec_slots() {
-  return ROUNDS >= 4 ? 3 : 6;
-}
-constexpr int kDecPipeThreads = (8 + kDecControl + 1) * 32;
-
-struct DecSlot {
-  uint32_t tile;     // kStopTile: none
-  uint32_t seg;
-  uint32_t nblk;     // blocks in the tile
-  uint32_t nel;      // elements of those blocks
-  uint64_t e0;       // first element of the tile (its segment's lo + 1 + blk0*L)
-  uint32_t first;    // first tile of its segment
-  uint32_t seed;     // q of the segment's element lo (first tile only)
-  uint32_t span0;    // region offset of span byte 0
-  uint32_t spanlen;  // staged span bytes
-  uint32_t sofs;     // slot byte offset of span byte 0
-  uint32_t pofs;     // slot word offset of the tile's first block offset
-  uint32_t seg_tile0;  // launch tile of its segment's first tile (the look-back stops there)
-  float eb;          // the field's bound
-  double ebd;        // float64 streams: the bound
-  float* y;          // the field's output (float64 streams: its doubles)
-  uint32_t* err;     // the field's error word
-};
-
-// Bytes of the block-offset area at the front of a slot.
-__host__ __device__ constexpr uint32_t dec_pos_bytes(uint32_t tb) { return 4 * tb + 32; }
-
-// Tile order of a decode pipeline launch.  A single field's launch is
-// cooperative (a.static_tiles), so all its CTAs are resident and CTA c takes
-// tiles c, c + grid, c + 2 grid, ...: the producer may run ahead as far as
-// its slots allow, and a tile's predecessors are the tiles the other CTAs hold
-// at the same time.  Batched launches, and a single field whose cooperative
-// launch was refused, draw tickets (a tile's predecessors have then started
-// before it).
-template <uint32_t L, uint32_t TB, int NS, bool BATCH, bool FM2>
-__device__ __forceinline__ void dec_producer(const DecArgs& a, uint8_t* slots, uint32_t slot_bytes, DecSlot* meta,
-                                             uint64_t* full, uint64_t* empty, uint32_t* s_epoch,
-                                             volatile uint32_t* s_stop_k, const volatile uint32_t* s_started) {
-  constexpr uint32_t PB = dec_pos_bytes(TB);
-  *s_epoch = *(volatile uint32_t*)&a.ls->epoch;
-  __threadfence();
-  // the plan of a single field and the region of the current segment, read once
-  uint32_t bad = 0, cseg = 0xFFFFFFFFu;
-  float eb = 0.0f;
-  double ebd = 0.0;
-  if (!BATCH) {
-    bad = a.f.plan->bad;
-    eb = a.f.plan->eb;
-    ebd = a.f.plan->ebd;
-  }
-  uint64_t R0 = 0;
-  uint32_t rlen = 0;
-  for (uint32_t k = 0, j = 0;; j++) {
-    const int s = (int)(k % NS);
-    if (k >= (uint32_t)NS) mbar_wait_or_flag(&empty[s], ((k / NS) - 1) & 1, a.err);
-    uint32_t tile;
-    if (BATCH || !a.static_tiles) {
-      // draw the ticket only once the compute warps have started the previous
-      // position: a tile's predecessors are then never more than a tile behind it
-      // in their work, which keeps the look-back short
-      for (uint32_t i = 0; i < kWaitLimit && *s_started < k; i++) __nanosleep(64);
-      tile = draw_ticket_persistent(a.ls, a.ntiles);
-    } else {
-      tile = blockIdx.x + j * gridDim.x;
-      if (tile >= a.ntiles) {
-        // the last CTA to stop advances the epoch (every CTA has read it)
-        const uint32_t t = atomicAdd(&a.ls->ticket, 1u);
-        if (t == gridDim.x - 1) {
-          a.ls->ticket = 0;
-          __threadfence();
-          atomicAdd(&a.ls->epoch, 1u);
-        }
-      }
-    }
-    DecSlot& m = meta[s];
-    if (tile >= a.ntiles) {
-      drain_copies<NS>(full, k);
-      m.tile = kStopTile;
-      *s_stop_k = k;
-      mbar_arrive(&full[s]);
-      return;
-    }
-    const DecField& fd = BATCH ? a.fields[a.tile_field[tile]] : a.f;
-    const Segments sg = fd.seg;
-    const DecTile dt = dec_tile(sg, tile - fd.tile_base, fd.tiles_per_seg, TB, FM2);
-    if (BATCH) bad = fd.plan->bad;
-    // nothing to write: a failed plan, an empty segment, a tile past its segment's blocks
-    // (fastmode1 keeps a segment's first tile for its seed)
-    if (bad || !dt.any || (dt.nblk == 0 && (FM2 || !dt.first))) continue;  // the slot stays free
-    const uint64_t lo = sg.lo(dt.seg), hi = sg.hi(dt.seg);
-    if (BATCH || dt.seg != cseg) {
-      R0 = fd.reg0[dt.seg];
-      rlen = (uint32_t)(fd.reg1[dt.seg] - R0);
-      cseg = dt.seg;
-    }
-    uint8_t* slot = slots + (size_t)s * slot_bytes;
-    m.seg = dt.seg;
-    m.seg_tile0 = fd.tile_base + (fd.tiles_per_seg ? dt.seg * fd.tiles_per_seg : 0u);
-    m.eb = BATCH ? fd.plan->eb : eb;
-    m.ebd = BATCH ? fd.plan->ebd : ebd;
-    m.y = fd.y;
-    m.err = fd.err;
-    m.nblk = dt.nblk;
-    m.first = dt.first;
-    m.e0 = FM2 ? lo + dt.blk0 * L : lo + 1 + dt.blk0 * L;  // fastmode2 blocks start with their seed
-    m.nel = dt.nblk ? (uint32_t)min((uint64_t)dt.nblk * L, hi - m.e0) : 0u;
-    m.seed = 0;
-    if (!FM2 && dt.first) {
-      const uint8_t* sp = fd.in + R0 - 4;  // the segment's 4-byte seed precedes its blocks
-      m.seed = (uint32_t)__ldg(sp) | ((uint32_t)__ldg(sp + 1) << 8) | ((uint32_t)__ldg(sp + 2) << 16) |
-               ((uint32_t)__ldg(sp + 3) << 24);
-    }
-    m.span0 = 0;
-    m.spanlen = 0;
-    m.sofs = PB;
-    m.pofs = 0;
-    uint32_t tx = 0;
-    uintptr_t p0 = 0, p1 = 0, q0 = 0, q1 = 0;
-    if (dt.nblk) {
-      const uint32_t* bp = fd.blkpos + seg_block_base(sg, dt.seg, FM2) + dt.blk0;
-      const uint32_t s0 = min(__ldg(bp), rlen);
-      uint32_t s1 = (uint32_t)min((uint64_t)rlen, (uint64_t)__ldg(bp + dt.nblk - 1) + a.maxsz);
-      if (s1 < s0) s1 = s0;
-      m.span0 = s0;
-      m.spanlen = min(s1 - s0, TB * a.maxsz);  // bounds a corrupt index to the slot
-      p0 = (uintptr_t)bp;
-      p1 = p0 + 4ull * dt.nblk;
-      m.pofs = (uint32_t)((p0 & 15) >> 2);
-      tx += stage_range(slot, reinterpret_cast<const uint8_t*>(fd.blkpos), 4 * fd.nblk_total, p0, p1);
-      q0 = (uintptr_t)(fd.in + R0 + s0);
-      q1 = q0 + m.spanlen;
-      m.sofs = PB + (uint32_t)(q0 & 15);
-      tx += stage_range(slot + PB, fd.in, fd.len, q0, q1);
-    }
-    m.tile = tile;
-    if (tx) {
-      fence_async_smem();
-      mbar_arrive_expect_tx(&full[s], tx);
-      stage_range_issue(slot, reinterpret_cast<const uint8_t*>(fd.blkpos), 4 * fd.nblk_total, p0, p1, &full[s]);
-      stage_range_issue(slot + PB, fd.in, fd.len, q0, q1, &full[s]);
-    } else {
-      mbar_arrive(&full[s]);
-    }
-    k++;
-  }
-}
-
-// All ones when byte k of w has its top bit set, else 0 (prmt's sign
-// replication; the __byte_perm intrinsic takes only the selector's low 3 bits).
-__device__ __forceinline__ uint32_t prmt_sign(uint32_t w, int k) {
-  uint32_t r;
-  switch (k) {
-    case 0: asm("prmt.b32 %0, %1, 0, 0x8888;" : "=r"(r) : "r"(w)); break;
-    case 1: asm("prmt.b32 %0, %1, 0, 0x9999;" : "=r"(r) : "r"(w)); break;
-    case 2: asm("prmt.b32 %0, %1, 0, 0xAAAA;" : "=r"(r) : "r"(w)); break;
-    default: asm("prmt.b32 %0, %1, 0, 0xBBBB;" : "=r"(r) : "r"(w)); break;
-  }
-  return r;
-}
-
-// Little-endian bytes [o, o+8) of shared array b as (lo, hi), from three
-// aligned 32-bit loads and two funnel shifts (reads b[o&~3 .. (o&~3)+12)).
-__device__ __forceinline__ void lds_le64(const uint8_t* b, uint32_t o, uint32_t& lo, uint32_t& hi) {
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(b + (o & ~3u));
-  const uint32_t sh = (o & 3u) * 8u;
-  const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
-  lo = __funnelshift_r(w0, w1, sh);
-  hi = __funnelshift_r(w1, w2, sh);
-}
-
-// The aligned middle of cta_dequant_store, compiled per 16-byte phase PH of
-// dst and per SPECIAL (eb not finite: the x86 NaN rule is applied): output
-// chunk c (4 floats) takes stage words [4c - PH, 4c - PH + 4), picked from
-// two aligned lines by fixed register moves.
-template <bool CODES, bool ACC, int PH, bool SPECIAL>
-__device__ __forceinline__ void cta_dequant_chunks(float* __restrict__ g0, const uint32_t* __restrict__ stage,
-                                                   uint32_t c0, uint32_t c1, uint32_t base, float eb, bool& wrap,
-                                                   uint32_t tid) {
-  auto dq = [eb](uint32_t q) -> float { return CODES ? __uint_as_float(q) : dequant(q, eb, SPECIAL); };
-  auto acc = [&wrap](float old, uint32_t q) -> float {  // old + q as int32 codes
-    const int32_t x = (int32_t)__float_as_uint(old), y = (int32_t)q;
-    const int32_t z = (int32_t)((uint32_t)x + (uint32_t)y);
-    wrap |= ((x ^ z) & (y ^ z)) < 0;
-    return __uint_as_float((uint32_t)z);
-  };
-  const uint4* s4 = reinterpret_cast<const uint4*>(stage);
-  // four chunks per thread per pass: their shared-memory loads are in flight together
-  constexpr int U = 4;
-  for (uint32_t cb = c0; cb < c1; cb += 256 * U) {
-    uint4 w[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const uint32_t c = min(cb + tid + 256 * u, c1 - 1);  // clamped: always a readable chunk
-      if constexpr (PH == 0) {
-        w[u] = s4[c];
-      } else {
-        const uint4 a = s4[c - 1], b = s4[c];  // stage words [4c-4, 4c+4)
-        const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        w[u] = make_uint4(v[4 - PH], v[5 - PH], v[6 - PH], v[7 - PH]);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const uint32_t c = cb + tid + 256 * u;
-      if (c < c1) {
-        float4 o;
-        if (ACC) {
-          const float4 p = reinterpret_cast<const float4*>(g0)[c];
-          o.x = acc(p.x, base + w[u].x);
-          o.y = acc(p.y, base + w[u].y);
-          o.z = acc(p.z, base + w[u].z);
-          o.w = acc(p.w, base + w[u].w);
-        } else {
-          o.x = dq(base + w[u].x);
-          o.y = dq(base + w[u].y);
-          o.z = dq(base + w[u].z);
-          o.w = dq(base + w[u].w);
-        }
-        reinterpret_cast<float4*>(g0)[c] = o;
-      }
-    }
-  }
-}
-
-// The 256 compute threads: y[e] = dequant(base + stage[e - e0]) for the
-// tile's nel elements starting at dst = y + e0; 16-byte stores for the aligned
-// middle (cta_dequant_chunks), plain stores at the ragged ends.  stage is
-// 16-byte aligned and readable for nel + 4 words.
-// CODES: the quantization codes themselves are stored (their bits), for the
-// homomorphic reduction; with ACC they are added to the codes already in dst
-// (wrapping int32; a wrap sets kErrQuantRange in *err).
-template <bool CODES = false, bool ACC = false>
-__device__ __forceinline__ void cta_dequant_store(float* __restrict__ dst, const uint32_t* __restrict__ stage,
-                                                  uint32_t nel, uint32_t base, float eb, bool ebsp,
-                                                  uint32_t* err = nullptr) {
-  auto dq = [eb, ebsp](uint32_t q) -> float { return CODES ? __uint_as_float(q) : dequant(q, eb, ebsp); };
-  bool wrap = false;
-  auto acc = [&wrap](float old, uint32_t q) -> float {  // old + q as int32 codes
-    const int32_t x = (int32_t)__float_as_uint(old), y = (int32_t)q;
-    const int32_t z = (int32_t)((uint32_t)x + (uint32_t)y);
-    wrap |= ((x ^ z) & (y ^ z)) < 0;
-    return __uint_as_float((uint32_t)z);
-  };
-  auto put = [&](float* p, uint32_t q) { *p = ACC ? acc(*p, q) : dq(q); };
-  const uint32_t tid = threadIdx.x;
-  if (nel == 0) return;
-  const uint32_t ph = (uint32_t)(((uintptr_t)dst >> 2) & 3);
-  float* g0 = dst - ph;  // 16-byte aligned
-  const uint32_t end = ph + nel;
-  const uint32_t c0 = (ph + 3) >> 2, c1 = end >> 2;  // whole float4 chunks [c0, c1)
-  if (c0 >= c1) {
-    if (tid < nel) put(g0 + ph + tid, base + stage[tid]);
-  } else {
-    if (tid < 4 * c0 - ph) put(g0 + ph + tid, base + stage[tid]);
-    if (tid >= 32 && tid - 32 < end - 4 * c1) put(g0 + 4 * c1 + tid - 32, base + stage[4 * c1 + tid - 32 - ph]);
-    if (!CODES && ebsp) {  // eb not finite
-      switch (ph) {
-        case 0: cta_dequant_chunks<CODES, ACC, 0, true>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-        case 1: cta_dequant_chunks<CODES, ACC, 1, true>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-        case 2: cta_dequant_chunks<CODES, ACC, 2, true>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-        default: cta_dequant_chunks<CODES, ACC, 3, true>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-      }
-    } else {
-      switch (ph) {
-        case 0: cta_dequant_chunks<CODES, ACC, 0, false>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-        case 1: cta_dequant_chunks<CODES, ACC, 1, false>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-        case 2: cta_dequant_chunks<CODES, ACC, 2, false>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-        default: cta_dequant_chunks<CODES, ACC, 3, false>(g0, stage, c0, c1, base, eb, wrap, tid); break;
-      }
-    }
-  }
-  if (ACC && wrap) atomicOr(err, kErrQuantRange);
-}
-
-// (double)q * eb of float64 data as bits: integer arithmetic for every eb
-// whose products stay normal (szp_f64.h), the FP64 multiply otherwise.
-struct DequantD {
-  uint64_t m, sgn;
-  uint32_t ef;
-  bool fast, special;
-  double eb;
-  __device__ __forceinline__ explicit DequantD(double e) : eb(e) {
-    const uint64_t u = f64i::bits_of(e);
-    fast = f64i::dequant_fast_ok(u);
-    special = !isfinite(e);
-    m = (u & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    ef = (uint32_t)(u >> 52) & 0x7FFu;
-    sgn = u & 0x8000000000000000ull;
-  }
-  __device__ __forceinline__ unsigned long long operator()(uint32_t q) const {
-    return fast ? f64i::dequant_bits((int32_t)q, m, ef, sgn) : f64i::bits_of(dequant(q, eb, special));
-  }
-};
-
-// cta_dequant_store for float64 data: y[e] = (double)(base + stage[e - e0]) * eb
-// for the tile's nel elements from dst = y + e0, 16-byte stores of two
-// results (the first result alone when dst is 8 bytes past a 16-byte
-// boundary), written as bits.
-__device__ __forceinline__ void cta_dequant_store_d(double* __restrict__ dst, const uint32_t* __restrict__ stage,
-                                                    uint32_t nel, uint32_t base, double eb) {
-  if (nel == 0) return;
-  const DequantD dq(eb);
-  const uint32_t tid = threadIdx.x;
-  unsigned long long* g = reinterpret_cast<unsigned long long*>(dst);
-  const uint32_t ph = (uint32_t)(((uintptr_t)dst >> 3) & 1);  // results before the first 16-byte boundary
-  if (ph && tid == 0) g[0] = dq(base + stage[0]);
-  const uint32_t n2 = (nel - ph) >> 1;
-  ulonglong2* g2 = reinterpret_cast<ulonglong2*>(g + ph);
-  for (uint32_t c = tid; c < n2; c += 256) {
-    const uint32_t e = ph + 2 * c;
-    g2[c] = make_ulonglong2(dq(base + stage[e]), dq(base + stage[e + 1]));
-  }
-  if (((nel - ph) & 1) && tid == 32) g[nel - 1] = dq(base + stage[nel - 1]);
-}
-
-// Control warp c: tiles c, c + kDecControl, ... of this CTA.  Finds each
-// tile's base q (the segment's seed plus the deltas of the tiles before it) and
-// hands it to the compute warps, which finish the tile.
-// Output kinds of the decode pipeline: floats, doubles (float64 streams,
-// dequantized in integer arithmetic, see DequantD), the int32 codes, or the
-// codes added to those already in y (the homomorphic reduction).
-enum { kOutFloat = 0, kOutDouble = 1, kOutCodes = 2, kOutCodesAdd = 3 };
-
-template <int NS, int NC, int OUT = kOutFloat>
-__device__ __forceinline__ void dec_control(int c, const DecArgs& a, const DecSlot* meta, const uint32_t* s_agg,
-                                            uint32_t* s_base, uint64_t* full, uint64_t* aggb, uint64_t* based,
-                                            const uint32_t* s_epoch, const volatile uint32_t* s_stop_k) {
-  const int lane = threadIdx.x & 31;
-  for (uint32_t k = (uint32_t)c;; k += NC) {
-    const int s = (int)(k % NS);
-    const uint32_t par = (k / NS) & 1;
-    if (!control_wait_full(&full[s], par, k, s_stop_k, a.err)) return;
-    const uint32_t tile = meta[s].tile;
-    if (tile >= a.ntiles) return;
-    const bool first = meta[s].first;
-    mbar_wait_or_flag(&aggb[s], par, a.err);
-    const uint32_t agg = s_agg[s];
-    const uint32_t epoch = *s_epoch;
-    uint32_t base;
-    if (first) {
-      base = meta[s].seed;
-      if (lane == 0) {
-        const float eb = meta[s].eb;
-        if (OUT == kOutDouble) {
-          reinterpret_cast<unsigned long long*>(meta[s].y)[meta[s].e0 - 1] = DequantD(meta[s].ebd)(base);
-        } else if (OUT == kOutCodes) {
-          meta[s].y[meta[s].e0 - 1] = __uint_as_float(base);
-        } else if (OUT == kOutCodesAdd) {
-          float* p = meta[s].y + meta[s].e0 - 1;
-          const int32_t x = (int32_t)__float_as_uint(*p), z = (int32_t)((uint32_t)x + base);
-          *p = __uint_as_float((uint32_t)z);
-          if (((x ^ z) & ((int32_t)base ^ z)) < 0) atomicOr(meta[s].err, kErrQuantRange);
-        } else {
-          meta[s].y[meta[s].e0 - 1] = dequant(base, eb, !isfinite(eb));
-        }
-      }
-    } else {
-      base = (uint32_t)lookback_sum(a.status, tile, meta[s].seg_tile0, epoch, a.err);
-      if (lane == 0) st_relaxed_u64(a.status + tile, make_status(epoch, kFlagInclusive, (uint32_t)(base + agg)));
-    }
-    if (lane == 0) {
-      s_base[s] = base;
-      mbar_arrive(&based[s]);
-    }
-    __syncwarp();
-  }
-}
-
-// OUT: what y holds (kOutFloat, kOutDouble: an array of doubles, kOutCodes:
-// int32 codes).
-template <int LPB, bool BATCH, int ROUNDS, bool FM2 = false, int OUT = kOutFloat>
-__global__ void __launch_bounds__(kDecPipeThreads, 2) decode_pipe(const __grid_constant__ DecArgs a,
-                                                                  uint32_t slot_bytes) {
-  constexpr int NS = dec_slots<ROUNDS>(), NC = kDecControl, WARPS = 8;
-  constexpr uint32_t DEFER = NS - 2;  // fastmode1: tiles between staging a tile and finishing it
-  // a control warp's next position must never share a slot phase it has not
-  // waited for (an mbarrier parity names one of two phases)
-  static_assert(NC <= NS, "more control warps than slots");
-  constexpr uint32_t L = 8 * LPB;
-  constexpr int BPR = 32 / LPB;
-  constexpr uint32_t TB = WARPS * ROUNDS * BPR;
-  constexpr uint32_t PB = dec_pos_bytes(TB);
-  extern __shared__ __align__(16) uint8_t s_slots[];
-  __shared__ DecSlot s_meta[NS];
-  __shared__ uint32_t s_agg[NS];
-  __shared__ uint32_t s_w[WARPS + 1];
-  __shared__ uint32_t s_epoch;
-  __shared__ volatile uint32_t s_stop_k;
-  __shared__ volatile uint32_t s_started;
-  __shared__ uint32_t s_base[NS];
-  __shared__ __align__(8) uint64_t s_full[NS], s_aggb[NS], s_based[NS], s_empty[NS];
-
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < NS) s_meta[threadIdx.x].tile = kStopTile;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < NS; s++) {
-      mbar_init(&s_full[s], 1);
-      mbar_init(&s_aggb[s], 1);
-      mbar_init(&s_based[s], 1);
-      mbar_init(&s_empty[s], 1);
-    }
-    s_stop_k = kStopTile;
-    s_started = 0;
-  }
-  __syncthreads();
-  if (warp == WARPS + NC) {
-    if (lane == 0)
-      dec_producer<L, TB, NS, BATCH, FM2>(a, s_slots, slot_bytes, s_meta, s_full, s_empty, &s_epoch, &s_stop_k,
-                                          &s_started);
-    return;
-  }
-  if (warp >= WARPS) {
-    // fastmode2 blocks carry their own seeds: no look-back, nothing to control
-    if (!FM2)
-      dec_control<NS, NC, OUT>(warp - WARPS, a, s_meta, s_agg, s_base, s_full, s_aggb, s_based, &s_epoch, &s_stop_k);
-    return;
-  }
-
-  // ---- compute warps ----
-  // Tile k is unpacked and staged, then tile k - DEFER (whose base the
-  // control warps have looked up meanwhile) is finished: base added,
-  // dequantized, stored.
-  const int sub = lane % LPB, grp = lane / LPB;
-  const uint32_t wfirst = (uint32_t)warp * ROUNDS * BPR;
-  auto finish = [&](uint32_t kp) {
-    const int sp_ = (int)(kp % NS);
-    mbar_wait_or_flag(&s_based[sp_], (kp / NS) & 1, a.err);
-    const float ebp = s_meta[sp_].eb;
-    const uint32_t* stage = reinterpret_cast<const uint32_t*>(s_slots + (size_t)sp_ * slot_bytes + PB);
-    if (OUT == kOutDouble) {
-      cta_dequant_store_d(reinterpret_cast<double*>(s_meta[sp_].y) + s_meta[sp_].e0, stage, s_meta[sp_].nel,
-                          s_base[sp_], s_meta[sp_].ebd);
-    } else {
-      cta_dequant_store<OUT >= kOutCodes, OUT == kOutCodesAdd>(s_meta[sp_].y + s_meta[sp_].e0, stage,
-                                                               s_meta[sp_].nel, s_base[sp_], ebp, !isfinite(ebp),
-                                                               s_meta[sp_].err);
-    }
-    compute_sync();  // every read of the slot is done
-    if (threadIdx.x == 0) mbar_arrive(&s_empty[sp_]);
-  };
-  for (uint32_t k = 0;; k++) {
-    const int s = (int)(k % NS);
-    const uint32_t par = (k / NS) & 1;
-    mbar_wait_or_flag(&s_full[s], par, a.err);
-    const uint32_t tile = s_meta[s].tile;
-    if (threadIdx.x == 0) s_started = k + 1;
-    if (tile >= a.ntiles) {
-      if (!FM2)  // fastmode2 tiles are finished at once
-        for (uint32_t j = k > DEFER ? k - DEFER : 0u; j < k; j++) finish(j);
-      return;
-    }
-    const uint32_t nblk = s_meta[s].nblk, nel = s_meta[s].nel, span0 = s_meta[s].span0;
-    const uint32_t spanlen = s_meta[s].spanlen;
-    uint8_t* slot = s_slots + (size_t)s * slot_bytes;
-    const uint8_t* sp = slot + s_meta[s].sofs;  // span byte i at sp[i]
-    const uint32_t* bpos = reinterpret_cast<const uint32_t*>(slot) + s_meta[s].pofs;
-
-    // ---- unpack deltas and prefix-add inside each lane ----
-    uint32_t pre[ROUNDS][8];
-    uint32_t lex[ROUNDS], rbase[ROUNDS];
-    uint32_t seedv[ROUNDS];  // fastmode2: each block's seed
-    uint32_t wtot = 0;
-    bool corrupt = false;
-    // FULL: a fastmode1 tile of TB whole blocks (every tile of a segment but
-    // its last); its rounds skip the per-block element counts
-    auto unpack = [&](auto fullc) {
-    constexpr bool FULL = decltype(fullc)::value;
-#pragma unroll
-    for (int r = 0; r < ROUNDS; r++) {
-      const uint32_t bt = wfirst + r * BPR + grp;
-      const uint32_t mblk = FULL ? L : (bt < nblk ? min(L, nel - bt * L) : 0u);
-      const uint32_t m = FM2 ? (mblk ? mblk - 1 : 0u) : mblk;  // values packed in the block
-      const uint32_t ml = FULL ? 8u : (m > 8u * sub ? min(8u, m - 8u * sub) : 0u);
-      uint32_t d[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++) d[j] = 0;
-      uint32_t off = 0, bc = 0;
-      seedv[r] = 0;
-      if (FULL) {
-        // a corrupt offset is kept inside the slot; a block of bit count b
-        // takes 1 + (L/8)(b+1) bytes (1 when b = 0)
-        off = min(bpos[bt] - span0, spanlen);
-        bc = sp[off];
-        if (bc > 33 || off + (bc ? 1 + (L / 8) * (bc + 1) : 1u) > spanlen) {
-          corrupt = true;
-          bc = 0;
-        }
-      } else if (FM2 && mblk) {
-        // fastmode2: the block's 4-byte seed, then its header (a one-element
-        // block has no header on the decode side, szpd_float.cc:483)
-        const uint32_t b0 = bpos[bt] - span0;
-        if (b0 + 4 > spanlen) {
-          corrupt = true;
-        } else {
-          seedv[r] = (uint32_t)sp[b0] | ((uint32_t)sp[b0 + 1] << 8) | ((uint32_t)sp[b0 + 2] << 16) |
-                     ((uint32_t)sp[b0 + 3] << 24);
-        }
-        off = b0 + 4;
-        if (m) {
-          bc = off < spanlen ? sp[off] : 255u;
-          if (bc > 33 || off + block_bytes(m, bc) > spanlen) {
-            corrupt = true;
-            bc = 0;
-          }
-        }
-      } else if (!FM2 && m) {
-        off = bpos[bt] - span0;
-        bc = off < spanlen ? sp[off] : 255u;
-        if (bc > 33 || off + block_bytes(m, bc) > spanlen) {
-          corrupt = true;
-          bc = 0;
-        }
-      }
-      constexpr uint32_t MF = FM2 ? L - 1 : L;  // values of a full block
-      if (__all_sync(0xffffffffu, (FULL || m == MF || m == 0) && bc <= 15)) {
-        // every block of the round is full and has at most one byte plane:
-        // the lane's plane and remainder bytes come from aligned word loads
-        // (fastmode2: L-1 values, the last lane's eighth is not one of them)
-        if (bc) {
-          constexpr uint32_t NSB = L / 8;  // sign bytes, ceil(MF / 8) either way
-          const uint32_t B = bc >> 3, rr = bc & 7;
-          const uint32_t ob = (uint32_t)(sp - s_slots) + off;  // the block in s_slots
-          const uint32_t sb = s_slots[ob + 1 + sub];             // sign bits, szp_TypeManager.cc:820-844
-          uint32_t lo, hi, plo = 0, phi = 0;
-          lds_le64(s_slots, ob + 1 + NSB + B * MF + rr * sub, lo, hi);  // remainder, szp_TypeManager.cc:122-434
-          if (B) lds_le64(s_slots, ob + 1 + NSB + 8 * sub, plo, phi);  // byte plane, szp_TypeManager.cc:36-52
-          const uint32_t t = __byte_perm(lo, 0, 0x0123);  // remainder bits 0..31, MSB first
-          const uint32_t t2 = __funnelshift_l(__byte_perm(hi, 0, 0x0123), t, 4 * rr);  // bits 4rr..
-          // byte k of sw0 (sw1) has the sign bit of value k (4 + k) as its top bit
-          const uint32_t sw0 = sb * 0x08040201u, sw1 = (sb << 4) * 0x08040201u;
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            // value j: its plane byte above its rr remainder bits, in one funnel shift
-            const uint32_t h = __byte_perm(j < 4 ? plo : phi, 0, 0x4440 + (j & 3));
-            const uint32_t v = __funnelshift_l((j < 4 ? t : t2) << (rr * (j & 3)), h, rr);
-            const uint32_t sg = prmt_sign(j < 4 ? sw0 : sw1, j & 3);  // 0 or all ones
-            d[j] = (FM2 && j == 7 && sub == LPB - 1) ? 0u : (v ^ sg) - sg;
-          }
-        }
-      } else if (m) {
-        if (bc && ml) {
-          const uint32_t ns = (m + 7) >> 3, B = bc >> 3, rr = bc & 7;
-          const uint32_t sb = sp[off + 1 + sub];  // sign bits, szp_TypeManager.cc:820-844
-          uint32_t hv[8];
-#pragma unroll
-          for (int j = 0; j < 8; j++) hv[j] = 0;
-          if (B) {  // byte planes, szp_TypeManager.cc:36-52
-            const uint8_t* q8 = sp + off + 1 + ns + 8 * B * sub;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-              if ((uint32_t)j < ml) {
-                uint32_t h = q8[j * B];
-                if (B > 1) h |= (uint32_t)q8[j * B + 1] << 8;
-                if (B > 2) h |= (uint32_t)q8[j * B + 2] << 16;
-                if (B > 3) h |= (uint32_t)q8[j * B + 3] << 24;
-                hv[j] = h << rr;
-              }
-            }
-          }
-          if (rr) {  // remainder bits, MSB first, szp_TypeManager.cc:122-434
-            const uint8_t* rp = sp + off + 1 + ns + B * m + rr * sub;
-            const uint32_t nb = (ml * rr + 7) >> 3;
-            uint64_t acc = 0;
-#pragma unroll
-            for (uint32_t kk = 0; kk < 7; kk++) acc = (acc << 8) | (uint64_t)(kk < nb ? rp[kk] : 0u);
-            // 56-bit window: field j occupies bits [56 - rr*(j+1), 56 - rr*j)
-            const uint32_t mask = (1u << rr) - 1u;
-#pragma unroll
-            for (int j = 0; j < 8; j++) hv[j] |= (uint32_t)(acc >> (56 - rr * (j + 1))) & mask;
-          }
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const uint32_t v = (uint32_t)j < ml ? hv[j] : 0u;
-            d[j] = ((sb >> (7 - j)) & 1u) ? 0u - v : v;
-          }
-        }
-      }
-      uint32_t run = 0;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        run += d[j];
-        pre[r][j] = run;
-      }
-      lex[r] = run;
-    }
-    };
-    if (!FM2 && nblk == TB && nel == TB * L) {
-      unpack(std::true_type{});
-    } else {
-      unpack(std::false_type{});
-    }
-    if constexpr (FM2) {
-      // every block restarts from its seed: a scan over the block's LPB lanes,
-      // the values staged, then the tile finished at once
-#pragma unroll
-      for (int r = 0; r < ROUNDS; r++) {
-        uint32_t incl = lex[r];
-#pragma unroll
-        for (int o = 1; o < LPB; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o, LPB);
-          if (sub >= o) incl += y;
-        }
-        lex[r] = incl - lex[r];
-      }
-      if (__any_sync(0xffffffffu, corrupt) && lane == 0) atomicOr(s_meta[s].err, kErrCorrupt);
-      compute_sync();  // every read of the span is done
-      uint32_t* stage = reinterpret_cast<uint32_t*>(slot + PB);
-#pragma unroll
-      for (int r = 0; r < ROUNDS; r++) {
-        const uint32_t bt = wfirst + r * BPR + grp;
-        const uint32_t mblk = bt < nblk ? min(L, nel - bt * L) : 0u;
-        const uint32_t m = mblk ? mblk - 1 : 0u;
-        const uint32_t ml = m > 8u * sub ? min(8u, m - 8u * sub) : 0u;
-        if (mblk && sub == 0) stage[bt * L] = seedv[r];
-        const uint32_t q0 = seedv[r] + lex[r];
-        const uint32_t k1 = bt * L + 1 + 8 * sub;
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-          if ((uint32_t)j < ml) stage[k1 + j] = q0 + pre[r][j];
-      }
-      compute_sync();
-      const float ebp = s_meta[s].eb;
-      if (OUT == kOutDouble) {
-        cta_dequant_store_d(reinterpret_cast<double*>(s_meta[s].y) + s_meta[s].e0, stage, nel, 0u, s_meta[s].ebd);
-      } else {
-        cta_dequant_store<OUT >= kOutCodes, OUT == kOutCodesAdd>(s_meta[s].y + s_meta[s].e0, stage, nel, 0u, ebp,
-                                                                 !isfinite(ebp), s_meta[s].err);
-      }
-      compute_sync();  // every read of the slot is done
-      if (threadIdx.x == 0) mbar_arrive(&s_empty[s]);
-      continue;
-    }
-    // the rounds' warp scans, interleaved: four independent shuffle chains
-    {
-      uint32_t incl[ROUNDS];
-#pragma unroll
-      for (int r = 0; r < ROUNDS; r++) incl[r] = lex[r];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-        for (int r = 0; r < ROUNDS; r++) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl[r], o);
-          if (lane >= o) incl[r] += y;
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < ROUNDS; r++) {
-        lex[r] = incl[r] - lex[r];
-        rbase[r] = wtot;
-        wtot += __shfl_sync(0xffffffffu, incl[r], 31);
-      }
-    }
-    if (__any_sync(0xffffffffu, corrupt) && lane == 0) atomicOr(s_meta[s].err, kErrCorrupt);
-
-    // ---- tile scan over the warps (its first barrier ends every read of the span) ----
-    if (lane == 0) s_w[warp] = wtot;
-    compute_sync();
-    uint32_t wexcl = 0, agg = 0;
-#pragma unroll
-    for (int w = 0; w < WARPS; w++) {
-      const uint32_t t = s_w[w];
-      wexcl += w < warp ? t : 0u;
-      agg += t;
-    }
-    if (threadIdx.x == 0) {
-      s_agg[s] = agg;
-      const bool first = s_meta[s].first;
-      const uint32_t v = first ? s_meta[s].seed + agg : agg;
-      st_relaxed_u64(a.status + tile, make_status(s_epoch, first ? kFlagInclusive : kFlagAggregate, v));
-      mbar_arrive(&s_aggb[s]);
-    }
-
-    // ---- stage the tile-relative prefix sums over the span ----
-    uint32_t* stage = reinterpret_cast<uint32_t*>(slot + PB);
-#pragma unroll
-    for (int r = 0; r < ROUNDS; r++) {
-      const uint32_t bt = wfirst + r * BPR + grp;
-      const uint32_t k0 = bt * L + 8 * sub;
-      const uint32_t ml = (bt < nblk && k0 < nel) ? min(8u, nel - k0) : 0u;
-      const uint32_t q0 = wexcl + rbase[r] + lex[r];
-      if (ml == 8) {
-        uint4* d4 = reinterpret_cast<uint4*>(stage + k0);
-        d4[0] = make_uint4(q0 + pre[r][0], q0 + pre[r][1], q0 + pre[r][2], q0 + pre[r][3]);
-        d4[1] = make_uint4(q0 + pre[r][4], q0 + pre[r][5], q0 + pre[r][6], q0 + pre[r][7]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-          if ((uint32_t)j < ml) stage[k0 + j] = q0 + pre[r][j];
-      }
-    }
-    compute_sync();  // staged; s_w is free for the next tile
-    if (k >= DEFER) finish(k - DEFER);
-  }
-}
-
 // Any blockSize, fastmode1 or fastmode2: one warp per block in 32-element
 // pieces.  fastmode1 decodes twice (totals, then values after the look-back).
 // V = float, or double for float64 streams (x' = (double)q * eb).
@@ -1614,36 +962,8 @@ __global__ void __launch_bounds__(WARPS * 32) decode_generic(const __grid_consta
   if (__any_sync(0xffffffffu, corrupt) && lane == 0) atomicOr(fd.err, kErrCorrupt);
 }
 
-static int dec_lanes_per_block(uint32_t L) {
-  switch (L) {
-    case 8: return 1;
-    case 16: return 2;
-    case 32: return 4;
-    case 64: return 8;
-    case 128: return 16;
-    case 256: return 32;
-    default: return 0;
-  }
-}
-
-uint32_t decode_blocks_per_tile(uint32_t L, uint32_t& bpw) {
-  int lpb = dec_lanes_per_block(L);
-  if (lpb) {
-    bpw = kDecRounds * (32 / lpb);
-    return kDecWarps * bpw;
-  }
-  uint32_t b = 2048u / (L < 32 ? 32u : L);
-  bpw = b < 1 ? 1 : (b > 8 ? 8 : b);
-  return kDecWarps * bpw;
-}
-
-size_t decode_smem_bytes(uint32_t L, uint32_t tb, bool fm2) {
-  if (fm2 || !dec_lanes_per_block(L)) return 0;
-  return (size_t)tb * max_block_bytes(L) + 64;
-}
-
 cudaError_t launch_dec_setup(const DecArgs& a, cudaStream_t st) {
-  dec_setup_kernel<false><<<1, 256, 0, st>>>(a);
+  dec_setup_kernel<false><<<1, 1024, 0, st>>>(a);  // a field of 0.5 GB has 7000 tickets to write
   return cudaGetLastError();
 }
 
@@ -1653,10 +973,10 @@ cudaError_t launch_dec_setup_batch(const DecArgs& a, uint32_t nfields, cudaStrea
   return cudaGetLastError();
 }
 
-template <bool FM2, bool BATCH>
+template <bool FM2>
 static cudaError_t launch_locate_t(const DecArgs& a, cudaStream_t st) {
   const size_t smem = locate_smem_bytes(a.super_chunk, a.overlap, a.maxsz);
-  auto k = locate_packs(a.super_chunk, a.maxsz) ? locate_kernel<FM2, BATCH, true> : locate_kernel<FM2, BATCH, false>;
+  auto k = locate_packs(a.super_chunk, a.maxsz) ? locate_kernel<FM2, true> : locate_kernel<FM2, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k<<<a.nlocate_ctas, kLocThreads, smem, st>>>(a);
@@ -1665,63 +985,10 @@ static cudaError_t launch_locate_t(const DecArgs& a, cudaStream_t st) {
 
 cudaError_t launch_locate(const DecArgs& a, cudaStream_t st) {
   if (a.nlocate_ctas == 0) return cudaSuccess;
-  return a.fm2 ? launch_locate_t<true, false>(a, st) : launch_locate_t<false, false>(a, st);
+  return a.fm2 ? launch_locate_t<true>(a, st) : launch_locate_t<false>(a, st);
 }
 
-cudaError_t launch_locate_batch(const DecArgs& a, cudaStream_t st) {
-  if (a.nlocate_ctas == 0) return cudaSuccess;
-  return launch_locate_t<false, true>(a, st);
-}
-
-// Bytes of one decode slot: the block offsets, then the stream span or the
-// staged prefix sums that replace it (read 16 bytes past their end).
-static uint32_t dec_slot_bytes(uint32_t L, uint32_t tb, uint32_t maxsz) {
-  const size_t span = (size_t)tb * maxsz + 32, stage = 4 * (size_t)tb * L + 32;
-  return (uint32_t)((dec_pos_bytes(tb) + (span > stage ? span : stage) + 15) & ~(size_t)15);
-}
-
-template <int LPB, bool BATCH = false, int ROUNDS = kDecRounds, bool FM2 = false, int OUT = kOutFloat>
-static cudaError_t launch_dec_lanes(const DecArgs& a, cudaStream_t st) {
-  auto k = decode_pipe<LPB, BATCH, ROUNDS, FM2, OUT>;
-  const uint32_t slot = dec_slot_bytes(8 * LPB, a.tb, a.maxsz);
-  const size_t smem = (size_t)dec_slots<ROUNDS>() * slot;
-  // resident CTAs of this instance, cached per device as (device + 1) << 32 | CTAs
-  static std::atomic<uint64_t> s_cache{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  uint64_t c = s_cache.load(std::memory_order_relaxed);
-  if ((c >> 32) != (uint64_t)dev + 1) {
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int occ = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kDecPipeThreads, smem);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    c = ((uint64_t)dev + 1) << 32 | (uint32_t)((occ < 1 ? 1 : occ) * sms);
-    s_cache.store(c, std::memory_order_relaxed);
-  }
-  const uint32_t cap = (uint32_t)c;
-  const uint32_t grid = a.ntiles < cap ? a.ntiles : cap;
-  if (grid == 0) return cudaSuccess;
-  if (!BATCH && a.static_tiles) {
-    // a single field's tiles are scheduled statically: its CTAs must all be
-    // resident, which a cooperative launch guarantees or refuses
-    DecArgs args = a;
-    uint32_t slot_arg = slot;
-    void* params[] = {&args, &slot_arg};
-    e = cudaLaunchCooperativeKernel((const void*)k, dim3(grid), dim3(kDecPipeThreads), params, smem, st);
-    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return e;
-    (void)cudaGetLastError();  // refused (a partitioned GPU): draw tickets instead
-  }
-  DecArgs args = a;
-  args.static_tiles = 0;
-  k<<<grid, kDecPipeThreads, smem, st>>>(args, slot);
-  return cudaGetLastError();
-}
-
-uint32_t decode_blocks_per_tile_f64(uint32_t L, uint32_t& bpw) {
+uint32_t decode_blocks_per_tile(uint32_t L, uint32_t& bpw) {
   const uint32_t b = 2048u / (L < 32 ? 32u : L);
   bpw = b < 1 ? 1 : (b > 8 ? 8 : b);
   return kDecWarps * bpw;
@@ -1736,117 +1003,13 @@ cudaError_t launch_decode_f64(const DecArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The fastmode pipelines for float64 streams (blockSize 8..256): a.f.y is the
-// output array of doubles.
-cudaError_t launch_decode_q(const DecArgs& a, cudaStream_t st) {
-  if (a.fm2) {
-    switch (dec_lanes_per_block(a.f.seg.L)) {
-      case 1: return launch_dec_lanes<1, false, kDecRounds, true, kOutDouble>(a, st);
-      case 2: return launch_dec_lanes<2, false, kDecRounds, true, kOutDouble>(a, st);
-      case 4: return launch_dec_lanes<4, false, kDecRounds, true, kOutDouble>(a, st);
-      case 8: return launch_dec_lanes<8, false, kDecRounds, true, kOutDouble>(a, st);
-      case 16: return launch_dec_lanes<16, false, kDecRounds, true, kOutDouble>(a, st);
-      case 32: return launch_dec_lanes<32, false, kDecRounds, true, kOutDouble>(a, st);
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  switch (dec_lanes_per_block(a.f.seg.L)) {
-    case 1: return launch_dec_lanes<1, false, kDecRounds, false, kOutDouble>(a, st);
-    case 2: return launch_dec_lanes<2, false, kDecRounds, false, kOutDouble>(a, st);
-    case 4: return launch_dec_lanes<4, false, kDecRounds, false, kOutDouble>(a, st);
-    case 8: return launch_dec_lanes<8, false, kDecRounds, false, kOutDouble>(a, st);
-    case 16: return launch_dec_lanes<16, false, kDecRounds, false, kOutDouble>(a, st);
-    case 32: return launch_dec_lanes<32, false, kDecRounds, false, kOutDouble>(a, st);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-// The fastmode pipelines writing the int32 codes to a.f.y, or adding them to
-// the codes there (accumulate); blockSize 8..256.
-template <int OUT>
-static cudaError_t launch_decode_codes_t(const DecArgs& a, cudaStream_t st) {
-  if (a.fm2) {
-    switch (dec_lanes_per_block(a.f.seg.L)) {
-      case 1: return launch_dec_lanes<1, false, kDecRounds, true, OUT>(a, st);
-      case 2: return launch_dec_lanes<2, false, kDecRounds, true, OUT>(a, st);
-      case 4: return launch_dec_lanes<4, false, kDecRounds, true, OUT>(a, st);
-      case 8: return launch_dec_lanes<8, false, kDecRounds, true, OUT>(a, st);
-      case 16: return launch_dec_lanes<16, false, kDecRounds, true, OUT>(a, st);
-      case 32: return launch_dec_lanes<32, false, kDecRounds, true, OUT>(a, st);
-      default: return cudaErrorInvalidValue;
-    }
-  }
-  switch (dec_lanes_per_block(a.f.seg.L)) {
-    case 1: return launch_dec_lanes<1, false, kDecRounds, false, OUT>(a, st);
-    case 2: return launch_dec_lanes<2, false, kDecRounds, false, OUT>(a, st);
-    case 4: return launch_dec_lanes<4, false, kDecRounds, false, OUT>(a, st);
-    case 8: return launch_dec_lanes<8, false, kDecRounds, false, OUT>(a, st);
-    case 16: return launch_dec_lanes<16, false, kDecRounds, false, OUT>(a, st);
-    case 32: return launch_dec_lanes<32, false, kDecRounds, false, OUT>(a, st);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-cudaError_t launch_decode_codes(const DecArgs& a, bool accumulate, cudaStream_t st) {
-  return accumulate ? launch_decode_codes_t<kOutCodesAdd>(a, st) : launch_decode_codes_t<kOutCodes>(a, st);
-}
-
 cudaError_t launch_decode(const DecArgs& a, cudaStream_t st) {
   if (a.fm2) {
-    switch (dec_lanes_per_block(a.f.seg.L)) {
-      case 1: return launch_dec_lanes<1, false, kDecRounds, true>(a, st);
-      case 2: return launch_dec_lanes<2, false, kDecRounds, true>(a, st);
-      case 4: return launch_dec_lanes<4, false, kDecRounds, true>(a, st);
-      case 8: return launch_dec_lanes<8, false, kDecRounds, true>(a, st);
-      case 16: return launch_dec_lanes<16, false, kDecRounds, true>(a, st);
-      case 32: return launch_dec_lanes<32, false, kDecRounds, true>(a, st);
-      default: break;
-    }
     decode_generic<kDecWarps, true><<<a.ntiles, kDecWarps * 32, 0, st>>>(a);
-    return cudaGetLastError();
+  } else {
+    decode_generic<kDecWarps, false><<<a.ntiles, kDecWarps * 32, 0, st>>>(a);
   }
-  switch (dec_lanes_per_block(a.f.seg.L)) {
-    case 1: return launch_dec_lanes<1>(a, st);
-    case 2: return launch_dec_lanes<2>(a, st);
-    case 4: return launch_dec_lanes<4>(a, st);
-    case 8: return launch_dec_lanes<8>(a, st);
-    case 16: return launch_dec_lanes<16>(a, st);
-    case 32: return launch_dec_lanes<32>(a, st);
-    default: break;
-  }
-  decode_generic<kDecWarps, false><<<a.ntiles, kDecWarps * 32, 0, st>>>(a);
   return cudaGetLastError();
-}
-
-// Sets the batched decompression kernels' shared-memory limits and caches
-// their grids without launching anything.
-cudaError_t prepare_decompress_batch() {
-  DecArgs a;
-  memset(&a, 0, sizeof a);
-  a.maxsz = max_block_bytes(32);
-  a.super_chunk = locate_super_bytes(a.maxsz);
-  a.overlap = locate_overlap_bytes(a.maxsz);
-  const size_t smem = locate_smem_bytes(a.super_chunk, a.overlap, a.maxsz);
-  cudaError_t e = cudaFuncSetAttribute(locate_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(locate_kernel<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  for (int r : {1, 2, 4}) {
-    if (e != cudaSuccess) return e;
-    a.tb = 8u * (uint32_t)r * 8u;
-    e = r == 1 ? launch_dec_lanes<4, true, 1>(a, 0) : r == 2 ? launch_dec_lanes<4, true, 2>(a, 0) : launch_dec_lanes<4, true, 4>(a, 0);
-  }
-  return e;
-}
-
-// Batched fastmode1 decode, blockSize 32, tiles of 8*rounds*8 blocks.
-cudaError_t launch_decode_batch(const DecArgs& a, uint32_t L, int rounds, cudaStream_t st) {
-  if (L != 32) return cudaErrorInvalidValue;
-  switch (rounds) {
-    case 1: return launch_dec_lanes<4, true, 1>(a, st);
-    case 2: return launch_dec_lanes<4, true, 2>(a, st);
-    case 4: return launch_dec_lanes<4, true, 4>(a, st);
-    default: return cudaErrorInvalidValue;
-  }
 }
 
 }  // namespace szp

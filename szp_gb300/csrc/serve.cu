@@ -147,7 +147,7 @@ struct Lane {
   std::vector<Req*> reqs;           // the group in flight
   std::vector<int> cidx, didx;      // their positions in the compress / decompress batch
   LaneScalars* misc = nullptr;      // device
-  Grow status, tables, htables, hresults, plans, blkpos, aux, sizes, errs;
+  Grow status, tables, htables, hresults, plans, map, sizes, errs;
 };
 
 }  // namespace
@@ -232,16 +232,15 @@ int launch_group(szp_gb300_server_s& s, Lane& ln) {
   CompressPlan cp;
   DecompressPlan dp;
   int rc = plan_compress(cf.data(), (int)cf.size(), L, T, tb, cp);
-  if (!rc) rc = plan_decompress(df.data(), (int)df.size(), L, T, tb, dp);
+  if (!rc) rc = plan_decompress(df.data(), (int)df.size(), L, T, dp);
   if (rc) return rc;
   const size_t nc = cf.size(), nd = df.size();
   // per-lane device buffers for this group
   SCU(ln.sizes.ensure(8 * (nc + 1), false, ln.st));
   SCU(ln.errs.ensure(4 * (nc + nd + 2), false, ln.st));
   SCU(ln.plans.ensure(dp.plan_stride * (nd + 1), false, ln.st));
-  SCU(ln.blkpos.ensure(4 * (dp.blocks + 1), false, ln.st));
-  SCU(ln.aux.ensure(sizeof(uint2) * (dp.locs + 1), false, ln.st));
-  const size_t words = std::max<uint64_t>(std::max(cp.tiles, dp.tiles), std::max<uint64_t>(dp.locs, 1));
+  SCU(ln.map.ensure(sizeof(uint4) * (dp.locs + 1), false, ln.st));
+  const size_t words = std::max<uint64_t>(cp.tiles, std::max<uint64_t>(2 * dp.locs, 1));
   if (words * 8 > ln.status.cap) {
     SCU(ln.status.ensure(words * 8, false, ln.st));
     SCU(cudaMemsetAsync(ln.status.p, 0, ln.status.cap, ln.st));  // fresh words must not look ready
@@ -250,11 +249,10 @@ int launch_group(szp_gb300_server_s& s, Lane& ln) {
   uint32_t* d_cerr = static_cast<uint32_t*>(ln.errs.p);
   uint32_t* d_derr = d_cerr + nc;
   place_compress(cp, d_sizes, d_cerr);
-  place_decompress(dp, static_cast<uint8_t*>(ln.plans.p), static_cast<uint32_t*>(ln.blkpos.p), d_derr);
+  place_decompress(dp, static_cast<uint8_t*>(ln.plans.p), d_derr);
   Packer pk;
   const size_t o_cf = pk.add(cp.fields), o_ctf = pk.add(cp.tile_field), o_it = pk.add(cp.item_field);
-  const size_t o_rs = pk.add(cp.rel), o_df = pk.add(dp.fields), o_dtf = pk.add(dp.tile_field);
-  const size_t o_lf = pk.add(dp.loc_field);
+  const size_t o_rs = pk.add(cp.rel), o_df = pk.add(dp.fields);
   SCU(ln.tables.ensure(pk.buf.size(), false, ln.st));
   SCU(ln.htables.ensure(pk.buf.size(), true));
   memcpy(ln.htables.p, pk.buf.data(), pk.buf.size());  // the lane's previous group has finished with it
@@ -274,10 +272,9 @@ int launch_group(szp_gb300_server_s& s, Lane& ln) {
   }
   if (nd) {
     DecArgs a;
-    args_decompress(a, dp, reinterpret_cast<DecField*>(tb_d + o_df), reinterpret_cast<uint32_t*>(tb_d + o_dtf),
-                    reinterpret_cast<uint32_t*>(tb_d + o_lf), static_cast<uint2*>(ln.aux.p), ln.misc->counters,
-                    static_cast<uint64_t*>(ln.status.p), &ln.misc->ls, &ln.misc->err, tb);
-    rc = issue_decompress(a, (uint32_t)nd, rounds, ln.st);
+    args_decompress(a, dp, reinterpret_cast<DecField*>(tb_d + o_df), static_cast<uint4*>(ln.map.p), ln.misc->counters,
+                    static_cast<uint64_t*>(ln.status.p), &ln.misc->ls, &ln.misc->err);
+    rc = issue_decompress(a, (uint32_t)nd, ln.st);
     if (rc) return rc;
   }
   // results: compressed sizes, per-field errors, the lane's error word
@@ -287,7 +284,7 @@ int launch_group(szp_gb300_server_s& s, Lane& ln) {
   SCU(cudaMemcpyAsync(hr + 8 * (nc + 1), d_cerr, 4 * (nc + nd), cudaMemcpyDeviceToHost, ln.st));
   SCU(cudaMemcpyAsync(hr + 8 * (nc + 1) + 4 * (nc + nd), &ln.misc->err, 4, cudaMemcpyDeviceToHost, ln.st));
   SCU(cudaEventRecord(ln.ev, ln.st));
-  host_count_launches((nc ? (cp.item_field.empty() ? 1 : 2) : 0) + (nd ? 3 : 0));
+  host_count_launches((nc ? (cp.item_field.empty() ? 1 : 2) : 0) + (nd ? 2 : 0));
   return SZP_GB300_OK;
 }
 
@@ -427,8 +424,7 @@ int szp_gb300_server_create(szp_gb300_server* out, const szp_gb300_server_config
     if (e == cudaSuccess) e = ln.sizes.ensure(8 * mb, false, ln.st);
     if (e == cudaSuccess) e = ln.errs.ensure(8 * mb, false, ln.st);
     if (e == cudaSuccess) e = ln.plans.ensure(512 * mb, false, ln.st);
-    if (e == cudaSuccess) e = ln.blkpos.ensure(16u << 20, false, ln.st);
-    if (e == cudaSuccess) e = ln.aux.ensure(1u << 20, false, ln.st);
+    if (e == cudaSuccess) e = ln.map.ensure(1u << 20, false, ln.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ln.st);
     if (e != cudaSuccess) return bad(e);
   }
@@ -552,7 +548,7 @@ void szp_gb300_server_destroy(szp_gb300_server s) {
   if (s->worker.joinable()) s->worker.join();
   for (Lane& ln : s->lanes) {
     if (ln.st) cudaStreamSynchronize(ln.st);
-    for (Grow* g : {&ln.status, &ln.tables, &ln.plans, &ln.blkpos, &ln.aux, &ln.sizes, &ln.errs})
+    for (Grow* g : {&ln.status, &ln.tables, &ln.plans, &ln.map, &ln.sizes, &ln.errs})
       g->free_it(false);
     ln.htables.free_it(true);
     ln.hresults.free_it(true);

@@ -27,28 +27,26 @@ struct CompressPlan {
 };
 
 struct DecompressPlan {
-  std::vector<DecField> fields;  // plan/reg0/reg1/chunk_base, blkpos, err: offsets until placed
-  std::vector<uint32_t> tile_field, loc_field;
-  uint64_t tiles = 0, locs = 0, blocks = 0;
+  std::vector<DecField> fields;  // plan/reg0/reg1/chunk_base, err: offsets until placed
+  uint64_t locs = 0;             // super-chunks, at most
   size_t plan_stride = 0;  // bytes of DecPlan + reg0[T] + reg1[T] + chunk_base[T+1] per field
 };
 
 int plan_compress(const szp_gb300_field* fl, int nf, int L, int T, uint32_t tb, CompressPlan& p);
 void place_compress(CompressPlan& p, unsigned long long* d_sizes, uint32_t* d_err);
-int plan_decompress(const szp_gb300_field* fl, int nf, int L, int T, uint32_t tb, DecompressPlan& p);
-void place_decompress(DecompressPlan& p, uint8_t* d_plans, uint32_t* d_blkpos, uint32_t* d_err);
+int plan_decompress(const szp_gb300_field* fl, int nf, int L, int T, DecompressPlan& p);
+void place_decompress(DecompressPlan& p, uint8_t* d_plans, uint32_t* d_err);
 
 // Launch arguments over placed tables.
 void args_compress(CompressArgs& a, RelBatchArgs& r, const CompressPlan& p, CompressField* d_fields,
                    const uint32_t* d_tile_field, const uint32_t* d_items, RelFieldState* d_state, uint64_t* status,
                    LaunchState* ls, uint32_t* err, uint32_t tb);
-void args_decompress(DecArgs& a, const DecompressPlan& p, const DecField* d_fields, const uint32_t* d_tile_field,
-                     const uint32_t* d_loc_field, uint2* aux, uint32_t* counters, uint64_t* status, LaunchState* ls,
-                     uint32_t* err, uint32_t tb);
+void args_decompress(DecArgs& a, const DecompressPlan& p, const DecField* d_fields, uint4* map, uint32_t* counters,
+                     uint64_t* status, LaunchState* ls, uint32_t* err);
 
 // The stages of one run.
 int issue_compress(const CompressArgs& a, const RelBatchArgs& r, uint32_t rel_grid, int rounds,
                    cudaStream_t st);
-int issue_decompress(const DecArgs& a, uint32_t nfields, int rounds, cudaStream_t st);
+int issue_decompress(const DecArgs& a, uint32_t nfields, cudaStream_t st);
 
 }  // namespace szp

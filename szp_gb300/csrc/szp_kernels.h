@@ -115,13 +115,10 @@ struct DecField {
   uint64_t* reg1;           // [T] absolute end of it (exclusive)
   uint32_t* blkpos;         // per block: header offset relative to its segment's region start
   uint64_t nblk_total;
-  float* y;                 // output
+  float* y;                 // output (decode_flow: of a.out_kind)
   double* yd;               // output of a float64 stream (decode_generic<.., double>)
-  uint32_t ntiles;          // decode tiles of this field
+  uint32_t ntiles;          // tiles of decode_generic
   uint32_t tiles_per_seg;
-  uint32_t tile_base;       // its first decode tile in the launch
-  uint32_t loc_base;        // its first locate ticket in the launch
-  uint32_t loc_ctas;        // locate tickets it may use
   uint32_t* err;            // this field's error word
 };
 
@@ -130,7 +127,7 @@ struct DecArgs {
   bool fm2;
   uint32_t hb;           // bytes of the stream's eb header: 4 (float) or 8 (double)
   uint32_t chunk;        // bytes per locate thread
-  uint32_t super_chunk;  // bytes per locate CTA (chunk * threads)
+  uint32_t super_chunk;  // bytes per locate CTA (chunk * threads); decode_flow: bytes per chunk
   uint32_t overlap;      // bytes walked before a CTA's region to find the header chain
   uint32_t maxsz;        // largest block (including a fastmode2 seed)
   uint2* aux;            // per locate ticket: (entry, exit) of its header chain
@@ -141,13 +138,21 @@ struct DecArgs {
   uint32_t ntiles;       // decode tiles of the launch
   uint32_t tb;
   uint32_t bpw;
-  uint32_t nlocate_ctas; // locate tickets of the launch (upper bound)
-  uint32_t static_tiles; // decode pipeline: CTA c takes tiles c, c + grid, ... (a cooperative launch)
-  // batched launches
-  const DecField* fields;
-  const uint32_t* tile_field;  // decode tile -> field
-  const uint32_t* loc_field;   // locate ticket -> field
+  uint32_t nlocate_ctas; // super-chunks of the launch (upper bound)
+  // decode_flow: what it writes, its tickets (written by dec_setup) and their number
+  int out_kind;
+  uint4* map;
+  uint32_t* ticket_total;
+  const DecField* fields;  // batched launches
 };
+
+// Stream bytes of a decode_flow super-chunk at most, and the bits of a ticket's
+// field number (its chunks stand above them).
+constexpr uint32_t kFlowSuper = 16384, kFlowFieldBits = 26, kFlowFieldMask = (1u << kFlowFieldBits) - 1;
+
+// What decode_flow writes: floats, doubles (float64 streams), the int32 codes,
+// or the codes added to those already there (the homomorphic reduction).
+enum { kOutFloat = 0, kOutDouble = 1, kOutCodes = 2, kOutCodesAdd = 3 };
 
 uint32_t compress_blocks_per_tile(uint32_t L, uint32_t& bpw);
 size_t compress_smem_bytes(uint32_t L, uint32_t tb);
@@ -186,19 +191,16 @@ uint32_t locate_chunk_bytes(uint32_t maxsz);
 uint32_t locate_super_bytes(uint32_t maxsz);
 uint32_t locate_overlap_bytes(uint32_t maxsz);
 size_t locate_smem_bytes(uint32_t super_chunk, uint32_t overlap, uint32_t maxsz);
-size_t decode_smem_bytes(uint32_t L, uint32_t tb, bool fm2);
 cudaError_t launch_dec_setup(const DecArgs& a, cudaStream_t st);
 cudaError_t launch_locate(const DecArgs& a, cudaStream_t st);
 cudaError_t launch_decode(const DecArgs& a, cudaStream_t st);
-uint32_t decode_blocks_per_tile_f64(uint32_t L, uint32_t& bpw);
 cudaError_t launch_decode_f64(const DecArgs& a, cudaStream_t st);
-cudaError_t launch_decode_q(const DecArgs& a, cudaStream_t st);      // a.f.y: the output doubles
-// a.f.y: the int32 codes (accumulate: added to the codes already there)
-cudaError_t launch_decode_codes(const DecArgs& a, bool accumulate, cudaStream_t st);
-// batched decompression (fastmode1, blockSize 32)
 cudaError_t launch_dec_setup_batch(const DecArgs& a, uint32_t nfields, cudaStream_t st);
-cudaError_t launch_locate_batch(const DecArgs& a, cudaStream_t st);
-cudaError_t launch_decode_batch(const DecArgs& a, uint32_t L, int rounds, cudaStream_t st);
+// blockSize 8..256, a power of two (decode_flow.cu); a batch is fastmode1, blockSize 32
+bool flow_supported(uint32_t L);
+uint32_t flow_chunk_bytes(uint32_t L);  // a super-chunk is 1 to 16 KB / this many of them
+cudaError_t launch_decode_flow(const DecArgs& a, cudaStream_t st);
+cudaError_t launch_decode_flow_batch(const DecArgs& a, cudaStream_t st);
 cudaError_t prepare_decompress_batch();
 
 // the multidimensional Lorenzo variant (lorenzo.cu)
