@@ -444,8 +444,13 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
     int32_t bseed[ROUNDS];  // fastmode2: each block's seed, in its first lane
     const uint32_t sh = 1 + g.d;  // slot index of tile element 0
     const uint32_t ph = sh & 3;   // its 16-byte phase (same for every lane: L % 8 == 0)
-    // every lane of every round holds 8 elements (never in fastmode2: a block has L-1 deltas)
-    const bool full = !FM2 && g.nblk == TB && g.nel == TB * L;
+    // the warp's blocks are whole: every lane of every round holds 8 elements
+    // (fastmode2: a block's last lane 7 deltas, `lone` keeps the eighth out).  A
+    // short tile works with masks only in the warps at the segment's end: every
+    // tile after it waits for its size (8192^2 values in 72 segments, fastmode1:
+    // 0.156 -> 0.120 ms on the blockSize-32 pipeline).
+    const bool full = ((uint32_t)warp + 1) * (ROUNDS * BPR * L) <= g.nel;
+    const bool lone = FM2 && sub == LPB - 1;
     // All rounds run on the fast quantization (exact while |x/eb| < 2^24); if
     // any lane met a larger value the whole tile is redone on the exact path,
     // so the common case has no per-round branch.
@@ -516,6 +521,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
       bseed[r] = prev;
       uint32_t sb = 0, lmax = 0;
       if (full) {
+        if (lone) q[7] = q[6];  // no eighth delta
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           const int32_t d = (int32_t)((uint32_t)q[j] - (uint32_t)prev);  // wrapping, as the compiled reference
@@ -612,20 +618,31 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
       for (int r = 0; r < ROUNDS; r++) {
         const uint32_t bc = rinfo[r] & 63;
         uint8_t* dst = s_tile + wexcl + (rinfo[r] >> 6);
+        if (FM2) {
+          if (sub == 0) {  // the block's seed, szp_float.cc:812-864
+            dst[0] = (uint8_t)bseed[r];
+            dst[1] = (uint8_t)((uint32_t)bseed[r] >> 8);
+            dst[2] = (uint8_t)((uint32_t)bseed[r] >> 16);
+            dst[3] = (uint8_t)((uint32_t)bseed[r] >> 24);
+          }
+          dst += 4;
+        }
         if (sub == 0) dst[0] = (uint8_t)bc;
         const uint32_t B = bc >> 3, rr = bc & 7;
-        constexpr uint32_t ns = L / 8;
+        constexpr uint32_t ns = L / 8;  // sign bytes; L - 1 signs take as many
         if (bc) dst[1 + sub] = (uint8_t)sgnb[r];
         if (__all_sync(0xffffffffu, B <= 1)) {
           if (B) {
             uint8_t* q8 = dst + 1 + ns + 8 * sub;
 #pragma unroll
-            for (int j = 0; j < 8; j++) q8[j] = (uint8_t)(vv[r][j] >> rr);
+            for (int j = 0; j < 8; j++)
+              if (j < 7 || !lone) q8[j] = (uint8_t)(vv[r][j] >> rr);
           }
         } else if (B) {
           uint8_t* q8 = dst + 1 + ns + 8 * B * sub;
 #pragma unroll
           for (int j = 0; j < 8; j++) {
+            if (j == 7 && lone) break;
             const uint32_t h = vv[r][j] >> rr;
             q8[j * B] = (uint8_t)h;
             if (B > 1) q8[j * B + 1] = (uint8_t)(h >> 8);
@@ -643,7 +660,8 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
           // 8*rr bits, element 0 first, moved to the top of 64 bits
           const uint64_t top = (((uint64_t)hi4 << (4 * rr)) | lo4) << (64 - 8 * rr);
           const uint32_t th = (uint32_t)(top >> 32), tl = (uint32_t)top;
-          uint8_t* rp = dst + 1 + ns + B * L + rr * sub;
+          // 7 deltas of rr bits end in the same byte as 8
+          uint8_t* rp = dst + 1 + ns + B * (FM2 ? L - 1 : L) + rr * sub;
           rp[0] = (uint8_t)(th >> 24);
           if (rr > 1) rp[1] = (uint8_t)(th >> 16);
           if (rr > 2) rp[2] = (uint8_t)(th >> 8);
@@ -1376,7 +1394,6 @@ cudaError_t launch_compress(const CompressArgs& a, bool fm2, cudaStream_t st) {
     switch (lanes_per_block(a.seg.L)) {
       case 1: return launch_lanes<1>(a, st);
       case 2: return launch_lanes<2>(a, st);
-      case 4: return launch_lanes<4>(a, st);
       case 8: return launch_lanes<8>(a, st);
       case 16: return launch_lanes<16>(a, st);
       case 32: return launch_lanes<32>(a, st);
@@ -1594,6 +1611,12 @@ cudaError_t launch_compress_q(const CompressArgs& a, bool fm2, cudaStream_t st) 
       default: return cudaErrorInvalidValue;
     }
   }
+  // float64 streams mostly hold 14 bits a value and more: their packed tiles are twice as
+  // large, the blockSize-32 pipeline's ring then holds two, and a tile waits for its
+  // position instead of for the next but one (2^25 values at REL 1e-6: 0.124 ms
+  // against 0.107 on the general pipeline; codes of float streams, 384^3 at REL 1e-3:
+  // 0.090 against 0.118)
+  if (a.qhb == 4 && compress32_supported(a)) return launch_compress32_q(a, st);
   switch (lanes_per_block(a.seg.L)) {
     case 1: return launch_lanes<1, false, kRounds, false, true>(a, st);
     case 2: return launch_lanes<2, false, kRounds, false, true>(a, st);

@@ -29,9 +29,15 @@
 //     rare, warp-uniform path (max >= 2^20);
 //   * two rounds' block sizes share one 32-bit scan (16-bit halves);
 //   * remainder bits accumulate by multiply-add (v < 2^r when bc < 8).
-// Tiles other than full ones (a segment's last, short tile) take a masked,
-// exact path.  Every other blockSize, fastmode2, float64 codes and the
-// batched launches stay on compress_pipe.
+//   * the ring is counted in 32 bits (64-bit remainders of its size took a
+//     tenth of a warp's instructions), the warps' totals are two warp
+//     reductions and one reduction per warp gives the packing's bounds:
+//     512^3 field at REL 1e-3, 0.204 -> 0.190 ms.
+// The warp that holds a segment's end takes a masked, exact path.  The same
+// kernel packs int32 codes under a float header (the homomorphic sum, the
+// Lorenzo variant).  Every other blockSize, fastmode2, float64 codes and the
+// batched launches stay on compress_pipe (with a batch's fields looked up tile
+// by tile this one took 0.57 ms for 256 fields against 0.47).
 #include <atomic>
 #include <cstring>
 
@@ -63,28 +69,28 @@ constexpr int kRecs = 16;
 static_assert(4 + kTB * 137 <= kRing, "the ring holds the largest tile");
 static_assert(kSlotBytes % 16 == 0 && kRing % 16 == 0, "16-byte-aligned regions");
 
+// A tile, written by the producer in place k % kRecs (a place is used again
+// long after the tile has been copied out).
 struct C32Meta {
-  uint64_t lo, hi, e0;  // segment element range; first element of the tile's first block
-  uint32_t tile;        // launch tile; kStopTile: no more tiles
-  uint32_t seg;         // segment
-  uint32_t nblk, nel;   // blocks of the tile and their elements
-  uint32_t d;           // slot float index of element e0 - 1
-  uint32_t first;       // first tile of its segment: the seed goes in front
-  uint32_t has_seg;     // the stream has elements
+  uint32_t tile;       // launch tile; kStopTile: no more tiles
+  uint32_t seg;        // segment
+  uint32_t nblk, nel;  // blocks of the tile and their elements
+  uint32_t d;          // slot float index of the element before the first block's first
+  uint32_t first;      // first tile of its segment (the stream has elements): the seed goes in front
 };
 
-// What the control warp needs of a tile, written by compute thread 0 once the
-// tile's packed size is known (before it is packed); the control warp's
-// stream position comes back in gpos.
+// What the control warp needs besides, written by compute thread 0 once the
+// tile's packed size is known (before it is packed); the address its bytes go
+// to comes back in dst.
 struct C32Rec {
-  uint64_t end;    // ring bytes allocated up to and including this tile
-  uint64_t gpos;   // stream position, written by the control warp (~0: does not fit)
-  uint32_t tile;   // launch tile
-  uint32_t seg;    // segment
-  uint32_t first;  // first tile of its segment (the stream has elements)
-  uint32_t agg;    // packed bytes
-  uint32_t rpos;   // ring offset of the packed bytes
+  uint8_t* dst;   // stream address, written by the control warp (null: does not fit)
+  uint32_t agg;   // packed bytes
+  uint32_t rpos;  // ring offset of the packed bytes
+  uint32_t span;  // ring bytes taken, with those skipped at the ring's end
 };
+
+// Barrier over the compute threads.
+__device__ __forceinline__ void c32_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kW * 32) : "memory"); }
 
 // Producer: one thread.  Draws tile tickets in order and, for each, stages
 // the input window [e0 - 1, e0 + nel) in a free slot (element e at slot float
@@ -99,7 +105,7 @@ __device__ __forceinline__ void c32_producer(const CompressArgs& a, uint8_t* slo
     const int s = (int)(k % kNS);
     if (k >= (uint32_t)kNS) mbar_wait_or_flag(&empty[s], ((k / kNS) - 1) & 1, a.err);
     const uint32_t tile = draw_ticket_persistent(a.ls, a.ntiles);
-    C32Meta& m = meta[s];
+    C32Meta& m = meta[k % kRecs];
     if (tile >= a.ntiles) {
       drain_copies<kNS>(full, k);
       m.tile = kStopTile;
@@ -121,14 +127,10 @@ __device__ __forceinline__ void c32_producer(const CompressArgs& a, uint8_t* slo
     const uint32_t nblk = nb > blk0 ? (uint32_t)min((uint64_t)kTB, nb - blk0) : 0u;
     const uint64_t e0 = lo + 1 + blk0 * kL;
     const uint32_t nel = nblk ? (uint32_t)min((uint64_t)nblk * kL, hi - e0) : 0u;
-    m.lo = lo;
-    m.hi = hi;
-    m.e0 = e0;
     m.seg = t;
     m.nblk = nblk;
     m.nel = nel;
-    m.first = ts == 0;
-    m.has_seg = sg.n > 0;
+    m.first = ts == 0 && sg.n > 0;
     m.d = 0;
     if (sg.n > 0 && (nblk || (ts == 0 && hi > lo))) {  // a lone seed still needs x[lo]
       const uintptr_t xa = (uintptr_t)a.x;
@@ -157,30 +159,37 @@ __device__ __forceinline__ void c32_producer(const CompressArgs& a, uint8_t* slo
 // (the eb header for the first tile, the decoupled look-back for the others),
 // the segment offset of a segment's first tile and the stream size after the
 // last tile.  The position goes back to the compute warps in the record.
-__device__ __forceinline__ void c32_control(const CompressArgs& a, C32Rec* rec, uint64_t* recb, uint64_t* based,
-                                            const uint32_t* s_epoch, const volatile uint32_t* s_stop_k, float eb) {
+template <bool QI>
+__device__ __forceinline__ void c32_control(const CompressArgs& a, const C32Meta* meta, C32Rec* rec, uint64_t* recb,
+                                            uint64_t* based, const uint32_t* s_epoch,
+                                            const volatile uint32_t* s_stop_k, float eb) {
   const int lane = threadIdx.x & 31;
-  const uint64_t head = 4 + 8ull * a.seg.T;
+  const uint32_t hb = QI ? a.qhb : 4;  // bytes of the eb header: float64 streams carry a double
   for (uint32_t k = 0;; k++) {
     const int p = (int)(k % kRecs);
     if (!control_wait_full(&recb[p], (k / kRecs) & 1, k, s_stop_k, a.err)) return;
+    const C32Meta& m = meta[p];
     C32Rec& r = rec[p];
-    const uint32_t tile = r.tile, agg = r.agg;
+    const uint32_t agg = r.agg;
     const uint32_t epoch = *s_epoch;
     uint64_t excl = 0;
-    if (tile == 0) {
-      write_header_warp(a.out, eb, a.seg, lane);
+    if (m.tile == 0) {
+      if (QI && hb == 8) {
+        write_header_warp(a.out, a.ebd_dev ? *a.ebd_dev : a.ebd, a.seg, lane);
+      } else {
+        write_header_warp(a.out, eb, a.seg, lane);
+      }
     } else {
-      excl = lookback_sum(a.status, tile, 0, epoch, a.err);
-      if (lane == 0) st_relaxed_u64(a.status + tile, make_status(epoch, kFlagInclusive, excl + agg));
+      excl = lookback_sum(a.status, m.tile, 0, epoch, a.err);
+      if (lane == 0) st_relaxed_u64(a.status + m.tile, make_status(epoch, kFlagInclusive, excl + agg));
     }
     if (lane == 0) {
-      const uint64_t gpos = head + excl;
+      const uint64_t gpos = hb + 8ull * a.seg.T + excl;
       const bool fits = gpos + agg <= a.cap;
-      if (tile == a.ntiles - 1) *a.out_size = gpos + agg;
-      if (r.first && fits) write_offset(a.out, r.seg, excl);
+      if (m.tile == a.ntiles - 1) *a.out_size = gpos + agg;
+      if (m.first && fits) write_offset(a.out, m.seg, excl, hb);
       if (!fits) atomicOr(a.err, kErrCapacity);
-      r.gpos = fits ? gpos : ~0ull;
+      r.dst = fits ? a.out + gpos : nullptr;
       mbar_arrive(&based[p]);
     }
     __syncwarp();
@@ -228,14 +237,6 @@ __device__ __forceinline__ void cta_store_span(uint8_t* __restrict__ dst, const 
   }
 }
 
-// max(m, |p|) that keeps a NaN (max.NaN), so one compare after the tile
-// catches both |x/eb| >= 2^24 and NaN inputs.
-__device__ __forceinline__ float maxabs_nan(float m, float p) {
-  float r;
-  asm("{\n .reg .f32 t;\n abs.f32 t, %2;\n max.NaN.f32 %0, %1, t;\n}" : "=f"(r) : "f"(m), "f"(p));
-  return r;
-}
-
 // Per lane and round: the 8 magnitudes, the sign byte (element 0 in bit 7),
 // the block's max and then bit count (the same in the block's 4 lanes).
 struct C32Analysis {
@@ -248,15 +249,16 @@ struct C32Analysis {
 // quantization q = trunc(x * inv) by the round-toward-zero float product,
 // exact while |x * inv| < 2^24; returns false when some element of the lane's
 // share (or the element before the warp's first) fails that or is NaN.
-template <int PH>
+template <int PH, bool QI>
 __device__ __forceinline__ bool c32_analyse_fast(const float* __restrict__ sx, uint32_t sh, float inv, int warp,
                                                  int lane, C32Analysis& an) {
   const int sub = lane & 3, grp = lane >> 2;
   float pm = 0.0f;
   // code of the element before the warp's first one
-  const float pb = __fmul_rz(sx[sh + (uint32_t)warp * (kR * 8 * kL) - 1], inv);
-  pm = maxabs_nan(pm, pb);
-  int32_t carry = __float2int_rz(pb);
+  const float xb = sx[sh + (uint32_t)warp * (kR * 8 * kL) - 1];
+  const float pb = __fmul_rz(xb, inv);
+  if (!QI) pm = maxabs_nan(pm, pb);
+  int32_t carry = QI ? __float_as_int(xb) : __float2int_rz(pb);
 #pragma unroll
   for (int r = 0; r < kR; r++) {
     const uint32_t k0 = ((uint32_t)(warp * kR + r) * 8 + grp) * kL + 8 * sub;
@@ -275,9 +277,13 @@ __device__ __forceinline__ bool c32_analyse_fast(const float* __restrict__ sx, u
     int32_t q[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      const float p = __fmul_rz(x[j], inv);
-      pm = maxabs_nan(pm, p);
-      q[j] = __float2int_rz(p);
+      if (QI) {
+        q[j] = __float_as_int(x[j]);
+      } else {
+        const float p = __fmul_rz(x[j], inv);
+        pm = maxabs_nan(pm, p);
+        q[j] = __float2int_rz(p);
+      }
     }
     int32_t prev = __shfl_up_sync(0xffffffffu, q[7], 1);
     if (lane == 0) prev = carry;
@@ -302,6 +308,7 @@ __device__ __forceinline__ bool c32_analyse_fast(const float* __restrict__ sx, u
 
 // Any tile, exact quantization and per-element masks (a segment's last tile,
 // a warp whose fast pass failed).  ml: elements of the lane in round r.
+template <bool QI>
 __device__ __forceinline__ void c32_analyse_exact(const float* __restrict__ sx, uint32_t sh, float inv,
                                                   const C32Meta& g, int warp, int lane, C32Analysis& an,
                                                   uint32_t& flags) {
@@ -313,11 +320,11 @@ __device__ __forceinline__ void c32_analyse_exact(const float* __restrict__ sx, 
     const uint32_t ml = (bt < g.nblk && k0 < g.nel) ? min(8u, g.nel - k0) : 0u;
     int32_t q[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) q[j] = (uint32_t)j < ml ? quantize(sx[sh + k0 + j], inv, flags) : 0;
+    for (int j = 0; j < 8; j++) q[j] = (uint32_t)j >= ml ? 0 : QI ? __float_as_int(sx[sh + k0 + j]) : quantize(sx[sh + k0 + j], inv, flags);
     // the element before the lane's first (a block's first lane takes it
     // from the block before, which may be another warp's)
     int32_t prev = __shfl_up_sync(0xffffffffu, q[7], 1);
-    if (sub == 0 && bt < g.nblk) prev = quantize(sx[sh + k0 - 1], inv, flags);
+    if (sub == 0 && bt < g.nblk) prev = QI ? __float_as_int(sx[sh + k0 - 1]) : quantize(sx[sh + k0 - 1], inv, flags);
     uint32_t sb = 0, lmax = 0;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
@@ -356,8 +363,20 @@ __device__ __forceinline__ void c32_pack_full(uint8_t* dst, const uint32_t (&v)[
     hi4 = (((v[0] & mk) * pw + (v[1] & mk)) * pw + (v[2] & mk)) * pw + (v[3] & mk);
     lo4 = (((v[4] & mk) * pw + (v[5] & mk)) * pw + (v[6] & mk)) * pw + (v[7] & mk);
     uint8_t* q8 = dst + 5 + 8 * B * sub;
-    for (uint32_t b = 0; b < bmax; b++) {
-      if (b < B) {
+    if (B == 1) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) q8[j] = (uint8_t)(v[j] >> rr);
+    } else if (bmax <= 2) {
+      if (B == 2) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const uint32_t h = v[j] >> rr;
+          q8[2 * j] = (uint8_t)h;
+          q8[2 * j + 1] = (uint8_t)(h >> 8);
+        }
+      }
+    } else {
+      for (uint32_t b = 0; b < B; b++) {
 #pragma unroll
         for (int j = 0; j < 8; j++) q8[j * B + b] = (uint8_t)((v[j] >> rr) >> (8 * b));
       }
@@ -409,11 +428,14 @@ __device__ __forceinline__ void c32_pack_masked(uint8_t* dst, const uint32_t (&v
   }
 }
 
+// QI: the input is int32 codes (float64 data quantized by a pass before, or the
+// homomorphic sum's).
+template <bool QI>
 __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_constant__ CompressArgs a) {
   extern __shared__ __align__(16) uint8_t s_dyn[];
   uint8_t* s_slots = s_dyn;                    // kNS input slots
   uint8_t* s_ring = s_dyn + kNS * kSlotBytes;  // kRing + kRingPad bytes
-  __shared__ C32Meta s_meta[kNS];
+  __shared__ C32Meta s_meta[kRecs];
   __shared__ C32Rec s_rec[kRecs];
   __shared__ uint32_t s_wtot[2][kW];  // compute warps' packed bytes, by tile parity
   __shared__ uint32_t s_thr[36];
@@ -424,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 36) s_thr[threadIdx.x] = a.thr.thr[threadIdx.x];
-  if (threadIdx.x < kNS) s_meta[threadIdx.x].tile = kStopTile;
+  if (threadIdx.x < kRecs) s_meta[threadIdx.x].tile = kStopTile;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kNS; s++) {
       mbar_init(&s_full[s], 1);
@@ -445,63 +467,76 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
     return;
   }
   if (warp == kW) {
-    c32_control(a, s_rec, s_recb, s_based, &s_epoch, &s_cstop_k, eb);
+    c32_control<QI>(a, s_meta, s_rec, s_recb, s_based, &s_epoch, &s_cstop_k, eb);
     return;
   }
 
   // ---- compute warps ----
-  const float inv = __fdiv_rn(1.0f, eb);
   const int sub = lane & 3, grp = lane >> 2;
   const uint32_t tid = threadIdx.x;
-  // Ring state, the same in every compute thread: bytes allocated and
-  // released, the next position to copy out, and the end of a copied tile
-  // whose space is released at the next barrier.
-  uint64_t rhead = 0, rtail = 0, pend_end = 0;
-  uint32_t ncopy = 0;
+  const float inv = __fdiv_rn(1.0f, eb);
+  // Ring state, the same in every compute thread: the next free offset, the
+  // bytes of tiles that are not released, those of copied tiles whose space is
+  // released at the next barrier, and the next position to copy out.
+  uint32_t rnext = 0, used = 0, pend = 0, ncopy = 0;
   // Copies position j out of the ring once the control warp has placed it.
   auto copy_out = [&](uint32_t j) {
     const int pj = (int)(j % kRecs);
     mbar_wait_or_flag(&s_based[pj], (j / kRecs) & 1, a.err);
-    const uint64_t gpos = s_rec[pj].gpos;
-    if (gpos != ~0ull) cta_store_span(a.out + gpos, s_ring + s_rec[pj].rpos, s_rec[pj].agg, tid);
-    pend_end = s_rec[pj].end;
+    uint8_t* const dst = s_rec[pj].dst;
+    if (dst) cta_store_span(dst, s_ring + s_rec[pj].rpos, s_rec[pj].agg, tid);
+    pend += s_rec[pj].span;
   };
   constexpr uint32_t kDefer = 2;  // tiles between packing a tile and copying it out
   for (uint32_t k = 0;; k++) {
     const int s = (int)(k % kNS);
     mbar_wait_or_flag(&s_full[s], (k / kNS) & 1, a.err);
-    const C32Meta g = s_meta[s];
+    const C32Meta& m = s_meta[k % kRecs];
+    C32Meta g;  // what the compute warps need
+    g.tile = m.tile;
+    g.nblk = m.nblk;
+    g.nel = m.nel;
+    g.d = m.d;
+    g.first = m.first;
     if (g.tile >= a.ntiles) {
       if (tid == 0) s_cstop_k = k;  // the control warp ends after the tiles before k
       // a tile's position does not mean it is packed: every warp has packed
       // tile k - 1 after this barrier (the tiles before it are older than
       // one barrier already)
-      compute_sync();
+      c32_sync();
       for (; ncopy < k; ncopy++) copy_out(ncopy);
       return;
     }
     const float* sx = reinterpret_cast<const float*>(s_slots + (size_t)s * kSlotBytes);
-    const bool seed = g.has_seg && g.first && g.hi > g.lo;  // the segment's seed element x[lo]
+    const bool seed = g.first;  // the segment's seed element x[lo]
     uint32_t flags = 0;
     int32_t seedv = 0;
-    if (seed && tid == 0) seedv = quantize(sx[g.d], inv, flags);  // window element 0
+    if (seed && tid == 0) seedv = QI ? __float_as_int(sx[g.d]) : quantize(sx[g.d], inv, flags);  // window element 0
 
     // ---- analysis ----
     C32Analysis an;
     const uint32_t sh = 1 + g.d;  // slot index of tile element 0
-    const bool full = g.nblk == kTB && g.nel == kTE;
-    bool exact = !full;
+    // the warp's share is whole blocks, or nothing, or holds the segment's end:
+    // only that warp of a short tile works with masks (a short tile holds up
+    // every tile after it until its size is known)
+    constexpr uint32_t kWE = kR * 8 * kL;  // elements per warp
+    const bool full = ((uint32_t)warp + 1) * kWE <= g.nel;
+    bool exact = !full && (uint32_t)warp * kWE < g.nel;
+    if (!full && !exact) {
+#pragma unroll
+      for (int r = 0; r < kR; r++) an.bc[r] = 0;
+    }
     if (full) {
       bool ok;
       switch (sh & 3) {
-        case 0: ok = c32_analyse_fast<0>(sx, sh, inv, warp, lane, an); break;
-        case 1: ok = c32_analyse_fast<1>(sx, sh, inv, warp, lane, an); break;
-        case 2: ok = c32_analyse_fast<2>(sx, sh, inv, warp, lane, an); break;
-        default: ok = c32_analyse_fast<3>(sx, sh, inv, warp, lane, an); break;
+        case 0: ok = c32_analyse_fast<0, QI>(sx, sh, inv, warp, lane, an); break;
+        case 1: ok = c32_analyse_fast<1, QI>(sx, sh, inv, warp, lane, an); break;
+        case 2: ok = c32_analyse_fast<2, QI>(sx, sh, inv, warp, lane, an); break;
+        default: ok = c32_analyse_fast<3, QI>(sx, sh, inv, warp, lane, an); break;
       }
       exact = !__all_sync(0xffffffffu, ok);
     }
-    if (exact) c32_analyse_exact(sx, sh, inv, g, warp, lane, an, flags);
+    if (exact) c32_analyse_exact<QI>(sx, sh, inv, g, warp, lane, an, flags);
     if (__any_sync(0xffffffffu, flags != 0) && lane == 0) atomicOr(a.err, kErrQuantRange);
     // block max -> bit count (int)log2f(max)+1 (szp_float.cc:253-262): the
     // exact width, one more at and above the libm thresholds (max >= 2^20)
@@ -546,16 +581,13 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
     // after the next tile's barrier, which every reader of it has passed
     uint32_t* wtot = s_wtot[k & 1];
     if (lane == 0) wtot[warp] = tot0 + tot1 + tot2 + tot3;
-    compute_sync();  // also ends every read of the input slot and of the last copied tile
-    rtail = pend_end;
+    c32_sync();  // also ends every read of the input slot and of the last copied tile
+    used -= pend;
+    pend = 0;
     const uint32_t front = seed ? 4u : 0u;
-    uint32_t wexcl = front, agg = front;
-#pragma unroll
-    for (int w = 0; w < kW; w++) {
-      const uint32_t t = wtot[w];
-      wexcl += w < warp ? t : 0u;
-      agg += t;
-    }
+    const uint32_t wt = lane < kW ? wtot[lane] : 0u;
+    const uint32_t agg = front + __reduce_add_sync(0xffffffffu, wt);
+    const uint32_t wexcl = front + __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
     if (tid == 0) {
       const bool head = g.tile == 0;  // the stream's first tile has no predecessor
       st_relaxed_u64(a.status + g.tile, make_status(s_epoch, head ? kFlagInclusive : kFlagAggregate, agg));
@@ -565,31 +597,31 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
     // ---- ring space: 16-byte-aligned and contiguous (a tile that would
     // wrap starts over at offset 0); when the older tiles leave too little,
     // they are copied out now ----
-    uint64_t start = rhead;
-    const uint32_t pos0 = (uint32_t)(start % kRing);
-    if (pos0 + agg > kRing) start += kRing - pos0;
-    const uint64_t end = start + ((agg + 15) & ~15u);
-    const uint32_t rpos = (uint32_t)(start % kRing);
-    while (end - rtail > kRing) {
-      if (ncopy == k) {  // nothing waits in the ring: the skipped bytes belong to no tile
-        rtail = start;
+    uint32_t rpos = rnext, skip = 0;
+    if (rpos + agg > kRing) {
+      skip = kRing - rpos;
+      rpos = 0;
+    }
+    const uint32_t need = (agg + 15) & ~15u;
+    while (used + skip + need > kRing) {
+      if (ncopy == k) {  // nothing waits in the ring
+        skip = 0;
         break;
       }
       copy_out(ncopy++);
-      compute_sync();  // the copied bytes are read before they are overwritten
-      rtail = pend_end;
+      c32_sync();  // the copied bytes are read before they are overwritten
+      used -= pend;
+      pend = 0;
     }
-    rhead = end;
+    used += skip + need;
+    rnext = rpos + need;
     uint8_t* out = s_ring + rpos;
     const int p = (int)(k % kRecs);
     if (tid == 0) {
       C32Rec& r = s_rec[p];
-      r.end = end;
-      r.tile = g.tile;
-      r.seg = g.seg;
-      r.first = g.has_seg && g.first;
       r.agg = agg;
       r.rpos = rpos;
+      r.span = skip + need;
       mbar_arrive(&s_recb[p]);  // the control warp can place the tile while it is packed
       if (seed) {
         out[0] = (uint8_t)seedv;
@@ -600,14 +632,14 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
     }
 
     // ---- pack into the ring ----
+    uint32_t top = 0;  // the warp's largest bit count
+#pragma unroll
+    for (int r = 0; r < kR; r++) top = max(top, an.bc[r]);
+    top = __reduce_max_sync(0xffffffffu, top);
     if (full) {
 #pragma unroll
-      for (int r = 0; r < kR; r++) {
-        const uint32_t bc = an.bc[r];
-        const uint32_t bmax = __reduce_max_sync(0xffffffffu, bc >> 3);
-        const uint32_t rmax = __reduce_max_sync(0xffffffffu, bc & 7);
-        c32_pack_full(out + wexcl + off[r], an.v[r], an.sb[r], bc, sub, bmax, rmax);
-      }
+      for (int r = 0; r < kR; r++)
+        c32_pack_full(out + wexcl + off[r], an.v[r], an.sb[r], an.bc[r], sub, top >> 3, top < 8 ? top : 7u);
     } else {
 #pragma unroll
       for (int r = 0; r < kR; r++) {
@@ -626,8 +658,9 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
 
 bool compress32_supported(const CompressArgs& a) { return a.seg.L == kL && a.fields == nullptr; }
 
-cudaError_t launch_compress32(const CompressArgs& a, cudaStream_t st) {
-  auto k = compress32_pipe;
+template <bool QI>
+static cudaError_t launch_c32(const CompressArgs& a, cudaStream_t st) {
+  auto k = compress32_pipe<QI>;
   const size_t smem = (size_t)kNS * kSlotBytes + kRing + kRingPad;
   // resident CTAs, cached per device as (device + 1) << 32 | CTAs
   static std::atomic<uint64_t> s_cache{0};
@@ -652,5 +685,8 @@ cudaError_t launch_compress32(const CompressArgs& a, cudaStream_t st) {
   k<<<grid, kThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
+
+cudaError_t launch_compress32(const CompressArgs& a, cudaStream_t st) { return launch_c32<false>(a, st); }
+cudaError_t launch_compress32_q(const CompressArgs& a, cudaStream_t st) { return launch_c32<true>(a, st); }
 
 }  // namespace szp

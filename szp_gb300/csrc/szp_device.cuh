@@ -57,6 +57,14 @@ __device__ __forceinline__ int32_t quantize(float x, float inv, uint32_t& flags)
   return quantize_slow(x, inv, flags);
 }
 
+// max(m, |p|) that keeps a NaN (max.NaN), so one compare after the tile
+// catches both |x/eb| >= 2^24 and NaN inputs.
+__device__ __forceinline__ float maxabs_nan(float m, float p) {
+  float r;
+  asm("{\n .reg .f32 t;\n abs.f32 t, %2;\n max.NaN.f32 %0, %1, t;\n}" : "=f"(r) : "f"(m), "f"(p));
+  return r;
+}
+
 // q = (int)(x * inv) for float64 data (szp_double.cc:209,228): the double
 // product rounds to nearest, the conversion truncates; out of range and NaN
 // give INT32_MIN like x86's cvttsd2si, and raise kErrQuantRange.

@@ -161,6 +161,7 @@ cudaError_t launch_compress(const CompressArgs& a, bool fm2, cudaStream_t st);
 // whenever it applies
 bool compress32_supported(const CompressArgs& a);
 cudaError_t launch_compress32(const CompressArgs& a, cudaStream_t st);
+cudaError_t launch_compress32_q(const CompressArgs& a, cudaStream_t st);  // int32 codes
 // float64 data: every blockSize on the one-warp-per-block kernels
 uint32_t compress_blocks_per_tile_f64(uint32_t L, uint32_t& bpw);
 size_t compress_smem_bytes_f64(uint32_t L, uint32_t tb);
