@@ -7,12 +7,14 @@
 // along x makes the packed values the 3-D Lorenzo residual.  The stream starts
 // with [nx][ny][nz] as u32 little-endian.  This file holds the passes around
 // the fastmode1 pipelines (which pack and unpack r as codes):
-//   lorenzo_codes_kernel  x -> r, and the 12-byte dims header (lorenzo_codes4_kernel:
-//                         the same by float4s)
-//   lorenzo_ysum_kernel   r -> r summed along y, in place
-//   lorenzo_zsum_kernel   ... summed along z and dequantized, in place
+//   lorenzo_codes_kernel  x -> r, and the 12-byte dims header
+//   lorenzo_zsum_kernel   r -> r summed along z, in place
+//   lorenzo_ysum_kernel   ... summed along y and dequantized, in place
 // The reference predicts along the flattened array only; this variant has no
 // reference code and is checked against the oracle's restatement.
+#include <cstring>
+#include <type_traits>
+
 #include "szp_device.cuh"
 #include "szp_kernels.h"
 
@@ -26,81 +28,87 @@ __device__ __forceinline__ float x86_dequant(uint32_t q, float eb, bool special)
   return special ? x86_nan_fix(r, f, eb) : r;
 }
 
-// x -> r: one CTA per row (j, k) at a time, rows blockIdx.x, + grid, ...
-// ((j, k) stepped without a division per row); each element quantizes itself
-// and its three neighbours in y and z (those rows were read moments before,
-// by this or a neighbouring CTA, and come from L2).
-__global__ void __launch_bounds__(256) lorenzo_codes_kernel(const LorenzoArgs a) {
+// x -> r.  A thread takes V neighbouring values of kCodeRows rows (and the row
+// above them) through `kz` planes, so that a value is quantized 5/4 times
+// instead of once for each of the four codes it enters: the differences along
+// y are taken in registers, and those along z against the plane before, which
+// the thread still holds.  V = 4 (16-byte loads and stores) where rows are
+// multiples of 4 values and x and r 16-byte aligned, else 1.
+// F2I runs at 16 lanes per clock and SM, an eighth of an add, and bound the
+// version that quantized each value's three neighbours again: 49 M values
+// (500 x 384 x 256) took 0.153 ms.
+constexpr int kCodeRows = 4;
+
+template <int V>
+__global__ void __launch_bounds__(256) lorenzo_codes_kernel(const LorenzoArgs a, uint32_t kz) {
   const float eb = a.eb_dev ? *a.eb_dev : a.eb;
   const float inv = __fdiv_rn(1.0f, eb);  // fastmode1's float inverse (szp_float.cc:185)
   uint32_t flags = 0;
-  const uint32_t nx = a.nx, ny = a.ny;
-  const uint64_t plane = (uint64_t)nx * ny, rows = (uint64_t)ny * a.nz;
-  const uint64_t G = gridDim.x;
-  const uint64_t gk = G / ny;
-  const uint32_t gj = (uint32_t)(G % ny);
-  uint64_t k = blockIdx.x / ny;
-  uint32_t j = (uint32_t)(blockIdx.x % ny);
-  for (uint64_t row = blockIdx.x; row < rows; row += G) {
-    const float* __restrict__ x0 = a.x + row * nx;
-    int32_t* __restrict__ r0 = a.r + row * nx;
-    for (uint32_t i = threadIdx.x; i < nx; i += blockDim.x) {
-      uint32_t v = (uint32_t)quantize(__ldg(x0 + i), inv, flags);
-      if (j) v -= (uint32_t)quantize(__ldg(x0 + i - nx), inv, flags);
-      if (k) v -= (uint32_t)quantize(__ldg(x0 + i - plane), inv, flags);
-      if (j && k) v += (uint32_t)quantize(__ldg(x0 + i - plane - nx), inv, flags);
-      r0[i] = (int32_t)v;
+  using XV = typename std::conditional<V == 4, float4, float>::type;
+  const uint32_t nxv = a.nx / V, ny = a.ny, nz = a.nz;
+  const uint64_t njb = (ny + kCodeRows - 1) / kCodeRows, nkc = (nz + kz - 1) / kz;
+  const uint64_t items = nxv * njb * nkc, plane = (uint64_t)nxv * ny;
+  const XV* __restrict__ xs = reinterpret_cast<const XV*>(a.x);
+  for (uint64_t it = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; it < items;
+       it += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)(it % nxv);
+    const uint64_t rest = it / nxv;
+    const uint32_t j0 = (uint32_t)(rest % njb) * kCodeRows, k0 = (uint32_t)(rest / njb) * kz;
+    const uint32_t k1 = (uint32_t)min((uint64_t)nz, (uint64_t)k0 + kz), rows = min((uint32_t)kCodeRows, ny - j0);
+    uint32_t wp[kCodeRows][V];  // y differences of the plane before
+#pragma unroll
+    for (int r = 0; r < kCodeRows; r++)
+#pragma unroll
+      for (int v = 0; v < V; v++) wp[r][v] = 0;
+    for (uint32_t k = k0 ? k0 - 1 : 0; k < k1; k++) {
+      const uint64_t at = k * plane + (uint64_t)j0 * nxv + i;
+      float x[kCodeRows + 1][V];
+#pragma unroll
+      for (int r = 0; r <= kCodeRows; r++) {
+        XV t{};  // row j0 - 1 + r
+        if (r ? (uint32_t)r <= rows : j0 > 0) t = __ldg(xs + at + (int64_t)(r - 1) * nxv);
+        memcpy(x[r], &t, sizeof t);
+      }
+      uint32_t q[kCodeRows + 1][V];
+      float pm = 0.0f;
+#pragma unroll
+      for (int r = 0; r <= kCodeRows; r++)
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+          const float p = __fmul_rz(x[r][v], inv);
+          pm = maxabs_nan(pm, p);
+          q[r][v] = (uint32_t)__float2int_rz(p);
+        }
+      if (!(pm < 16777216.0f)) {  // a value whose float product is not exact, or NaN
+#pragma unroll
+        for (int r = 0; r <= kCodeRows; r++)
+#pragma unroll
+          for (int v = 0; v < V; v++)
+            if (r ? (uint32_t)r <= rows : j0 > 0) q[r][v] = (uint32_t)quantize(x[r][v], inv, flags);
+      }
+      if (j0 == 0) {
+#pragma unroll
+        for (int v = 0; v < V; v++) q[0][v] = 0;
+      }
+#pragma unroll
+      for (int r = 0; r < kCodeRows; r++) {
+        int32_t o[V];
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+          const uint32_t w = q[r + 1][v] - q[r][v];
+          o[v] = (int32_t)(w - wp[r][v]);
+          wp[r][v] = w;
+        }
+        if (k >= k0 && (uint32_t)r < rows) {
+          int32_t* dst = a.r + (at + (uint64_t)r * nxv) * V;
+          if constexpr (V == 4) {
+            *reinterpret_cast<int4*>(dst) = make_int4(o[0], o[1], o[2], o[3]);
+          } else {
+            dst[0] = o[0];
+          }
+        }
+      }
     }
-    j += gj;
-    k += gk;
-    if (j >= ny) {
-      j -= ny;
-      k++;
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x < 12) {
-    const uint32_t d[3] = {a.nx, a.ny, a.nz};
-    a.head[threadIdx.x] = (uint8_t)(d[threadIdx.x >> 2] >> (8 * (threadIdx.x & 3)));
-  }
-  if (__any_sync(0xffffffffu, flags != 0) && (threadIdx.x & 31) == 0) atomicOr(a.err, kErrQuantRange);
-}
-
-// The same codes, 4 elements per thread: rows of nx = 4 * nx4 values, x and r
-// 16-byte aligned, n / 4 below 2^32.  A flat grid-stride over the float4s of
-// the field; each takes its row's (j, k) by two 32-bit divisions and loads its
-// three neighbours as float4s (from L2: the grid covers several planes at once).
-__global__ void __launch_bounds__(256) lorenzo_codes4_kernel(const LorenzoArgs a) {
-  const float eb = a.eb_dev ? *a.eb_dev : a.eb;
-  const float inv = __fdiv_rn(1.0f, eb);
-  uint32_t flags = 0;
-  const uint32_t nx4 = a.nx >> 2, ny = a.ny;
-  const uint32_t plane4 = nx4 * ny;
-  const uint32_t total = plane4 * a.nz;
-  const float4* __restrict__ x4 = reinterpret_cast<const float4*>(a.x);
-  int4* __restrict__ r4 = reinterpret_cast<int4*>(a.r);
-  auto q4 = [&](float4 v) {
-    return make_int4(quantize(v.x, inv, flags), quantize(v.y, inv, flags), quantize(v.z, inv, flags),
-                     quantize(v.w, inv, flags));
-  };
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i64 < total; i64 += stride) {
-    const uint32_t it = (uint32_t)i64;
-    const uint32_t row = it / nx4, j = row % ny, k = row / ny;
-    const int4 c = q4(__ldg(x4 + it));
-    uint32_t v0 = (uint32_t)c.x, v1 = (uint32_t)c.y, v2 = (uint32_t)c.z, v3 = (uint32_t)c.w;
-    if (j) {
-      const int4 p = q4(__ldg(x4 + it - nx4));
-      v0 -= (uint32_t)p.x; v1 -= (uint32_t)p.y; v2 -= (uint32_t)p.z; v3 -= (uint32_t)p.w;
-    }
-    if (k) {
-      const int4 p = q4(__ldg(x4 + it - plane4));
-      v0 -= (uint32_t)p.x; v1 -= (uint32_t)p.y; v2 -= (uint32_t)p.z; v3 -= (uint32_t)p.w;
-    }
-    if (j && k) {
-      const int4 p = q4(__ldg(x4 + it - plane4 - nx4));
-      v0 += (uint32_t)p.x; v1 += (uint32_t)p.y; v2 += (uint32_t)p.z; v3 += (uint32_t)p.w;
-    }
-    r4[it] = make_int4((int32_t)v0, (int32_t)v1, (int32_t)v2, (int32_t)v3);
   }
   if (blockIdx.x == 0 && threadIdx.x < 12) {
     const uint32_t d[3] = {a.nx, a.ny, a.nz};
@@ -110,54 +118,56 @@ __global__ void __launch_bounds__(256) lorenzo_codes4_kernel(const LorenzoArgs a
 }
 
 // In-place running sums of q along a line of `len` elements `stride` apart,
-// starting at p; eight loads in flight before their sums are stored.
-// DEQ: the sums are dequantized ((float)q * eb, szpd_float.cc:67,86,112) and
-// stored as floats.
+// starting at p; 16 loads in flight before their sums are stored (8 left a
+// third of the bandwidth unused: a column per thread is all the parallelism a
+// field has).  DEQ: the sums are dequantized ((float)q * eb,
+// szpd_float.cc:67,86,112) and stored as floats.
 template <bool DEQ>
 __device__ __forceinline__ void lorenzo_line(int32_t* __restrict__ p, uint64_t stride, uint32_t len, float eb,
                                              bool special) {
+  constexpr int U = 16;
   uint32_t run = 0;
+  auto put = [&](uint64_t at) {
+    if (DEQ) {
+      reinterpret_cast<float*>(p)[at] = x86_dequant(run, eb, special);
+    } else {
+      p[at] = (int32_t)run;
+    }
+  };
   uint32_t j = 0;
-  for (; j + 8 <= len; j += 8) {
-    uint32_t v[8];
+  for (; j + U <= len; j += U) {
+    uint32_t v[U];
 #pragma unroll
-    for (int u = 0; u < 8; u++) v[u] = (uint32_t)p[(j + u) * stride];
+    for (int u = 0; u < U; u++) v[u] = (uint32_t)p[(j + u) * stride];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
+    for (int u = 0; u < U; u++) {
       run += v[u];
-      if (DEQ) {
-        reinterpret_cast<float*>(p)[(j + u) * stride] = x86_dequant(run, eb, special);
-      } else {
-        p[(j + u) * stride] = (int32_t)run;
-      }
+      put((j + u) * stride);
     }
   }
   for (; j < len; j++) {
     run += (uint32_t)p[j * stride];
-    if (DEQ) {
-      reinterpret_cast<float*>(p)[j * stride] = x86_dequant(run, eb, special);
-    } else {
-      p[j * stride] = (int32_t)run;
-    }
+    put(j * stride);
   }
 }
 
-// One thread per (k, i): sums along y.
-__global__ void __launch_bounds__(256) lorenzo_ysum_kernel(const LorenzoArgs a) {
-  const uint64_t cols = (uint64_t)a.nx * a.nz, plane = (uint64_t)a.nx * a.ny;
-  for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = c % a.nx, k = c / a.nx;
-    lorenzo_line<false>(a.q + k * plane + i, a.nx, a.ny, 0.0f, false);
-  }
-}
-
-// One thread per (j, i): sums along z, then dequantizes in place.
-__global__ void __launch_bounds__(256) lorenzo_zsum_kernel(const LorenzoArgs a) {
-  const float eb = *a.eb_dev;
-  const bool special = !isfinite(eb);
+// One thread per (j, i): sums along z.
+__global__ void __launch_bounds__(64) lorenzo_zsum_kernel(const LorenzoArgs a) {
   const uint64_t cols = (uint64_t)a.nx * a.ny;
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += (uint64_t)gridDim.x * blockDim.x)
-    lorenzo_line<true>(a.q + c, cols, a.nz, eb, special);
+    lorenzo_line<false>(a.q + c, cols, a.nz, 0.0f, false);
+}
+
+// One thread per (k, i): sums along y, then dequantizes in place; the last
+// planes first, whose sums along z are still in L2 (of 126 MB).
+__global__ void __launch_bounds__(64) lorenzo_ysum_kernel(const LorenzoArgs a) {
+  const float eb = *a.eb_dev;
+  const bool special = !isfinite(eb);
+  const uint64_t cols = (uint64_t)a.nx * a.nz, plane = (uint64_t)a.nx * a.ny;
+  for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = c % a.nx, k = a.nz - 1 - c / a.nx;
+    lorenzo_line<true>(a.q + k * plane + i, a.nx, a.ny, eb, special);
+  }
 }
 
 static uint32_t lorenzo_grid(uint64_t items, uint32_t per_cta, uint32_t cap) {
@@ -166,21 +176,27 @@ static uint32_t lorenzo_grid(uint64_t items, uint32_t per_cta, uint32_t cap) {
 }
 
 cudaError_t launch_lorenzo_codes(const LorenzoArgs& a, uint32_t sm_count, cudaStream_t st) {
-  const uint64_t n4 = (uint64_t)a.nx * a.ny * a.nz / 4;
-  if ((a.nx & 3) == 0 && n4 > 0 && n4 < (1ull << 32) && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.r & 15) == 0) {
-    lorenzo_codes4_kernel<<<lorenzo_grid(n4, 256, 8 * sm_count), 256, 0, st>>>(a);
+  const bool v4 = (a.nx & 3) == 0 && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.r & 15) == 0;
+  // columns of kCodeRows rows; planes are split among threads until there are
+  // 1024 threads per SM, but not below 8 (the plane before the first is read too)
+  const uint64_t cols = (uint64_t)(v4 ? a.nx / 4 : a.nx) * ((a.ny + kCodeRows - 1) / kCodeRows);
+  uint32_t kz = a.nz ? a.nz : 1;
+  while (kz > 8 && cols * ((a.nz + kz - 1) / kz) < 1024ull * sm_count) kz = (kz + 1) / 2;
+  const uint64_t items = cols * ((a.nz + kz - 1) / kz);
+  if (v4) {
+    lorenzo_codes_kernel<4><<<lorenzo_grid(items, 256, 1u << 30), 256, 0, st>>>(a, kz);
   } else {
-    lorenzo_codes_kernel<<<lorenzo_grid((uint64_t)a.ny * a.nz, 1, 8 * sm_count), 256, 0, st>>>(a);
+    lorenzo_codes_kernel<1><<<lorenzo_grid(items, 256, 1u << 30), 256, 0, st>>>(a, kz);
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_lorenzo_inverse(const LorenzoArgs& a, uint32_t sm_count, cudaStream_t st) {
   if ((uint64_t)a.nx * a.ny * a.nz == 0) return cudaSuccess;
-  lorenzo_ysum_kernel<<<lorenzo_grid((uint64_t)a.nx * a.nz, 256, 16 * sm_count), 256, 0, st>>>(a);
+  lorenzo_zsum_kernel<<<lorenzo_grid((uint64_t)a.nx * a.ny, 64, 32 * sm_count), 64, 0, st>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  lorenzo_zsum_kernel<<<lorenzo_grid((uint64_t)a.nx * a.ny, 256, 16 * sm_count), 256, 0, st>>>(a);
+  lorenzo_ysum_kernel<<<lorenzo_grid((uint64_t)a.nx * a.nz, 64, 32 * sm_count), 64, 0, st>>>(a);
   return cudaGetLastError();
 }
 
