@@ -532,7 +532,7 @@ int decompress_launch(Workspace& w, const DecompressJob& j, cudaStream_t st) {
   f.chunk_base = reinterpret_cast<uint32_t*>(f.reg1 + j.T);
   a.chunk = C;
   a.super_chunk = SC;
-  a.overlap = g_overlap >= 0 ? (uint32_t)g_overlap : locate_overlap_bytes(maxsz);
+  a.overlap = g_overlap >= 0 ? (uint32_t)g_overlap : flow ? 65536u : locate_overlap_bytes(maxsz);
   a.maxsz = maxsz;
   a.aux = w.walks.as<uint2>();
   a.counters = dm->verify;

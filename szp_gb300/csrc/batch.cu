@@ -353,12 +353,11 @@ void args_compress(CompressArgs& a, RelBatchArgs& r, const CompressPlan& p, Comp
 
 void args_decompress(DecArgs& a, const DecompressPlan& p, const DecField* d_fields, uint4* map, uint32_t* counters,
                      uint64_t* status, LaunchState* ls, uint32_t* err) {
-  const uint32_t maxsz = max_block_bytes(kBatchL);
   memset(&a, 0, sizeof a);
   a.fm2 = false;
   a.super_chunk = flow_chunk_bytes(kBatchL);
-  a.overlap = locate_overlap_bytes(maxsz);
-  a.maxsz = maxsz;
+  a.overlap = 65536u;  // as much as the kernel stages
+  a.maxsz = max_block_bytes(kBatchL);
   a.counters = counters;
   a.status = status;
   a.ls = ls;

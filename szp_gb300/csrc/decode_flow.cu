@@ -63,6 +63,7 @@ struct Shape {
   static constexpr uint32_t C = LPB <= 4 ? 1024 : 256 * LPB;       // bytes per chunk (a walking lane)
   static constexpr uint32_t NB = 16384 / C;                        // chunks
   static constexpr uint32_t W = C / 2;                             // bytes walked before a chunk to find its entry
+  static constexpr uint32_t LEAD2 = W < 4096 ? 4096 : W;           // bytes staged before a super-chunk, fastmode2
   static constexpr uint32_t CAPL = 2048 / NB;                      // blocks a lane notes while it walks
   static constexpr uint32_t KCAP = LPB <= 4 ? 1536 : 512;          // blocks listed at a time
 };
@@ -78,7 +79,7 @@ __host__ __device__ constexpr uint32_t flow_maxsz() {
 // phase, the last block's rest, and what loads read past a block's end.
 template <int LPB, bool FM2>
 __host__ __device__ constexpr uint32_t flow_smem() {
-  return 16 + Shape<LPB>::W + Shape<LPB>::C * Shape<LPB>::NB + flow_maxsz<LPB, FM2>() + 8 + 32;
+  return 16 + (FM2 ? Shape<LPB>::LEAD2 : Shape<LPB>::W) + Shape<LPB>::C * Shape<LPB>::NB + flow_maxsz<LPB, FM2>() + 8 + 32;
 }
 
 // The super-chunk a CTA is working on.
@@ -97,6 +98,13 @@ struct FlowTile {
   uint32_t align;           // shared-memory offset of the first staged byte
   uint32_t seed;            // q of the segment's first element (fastmode1, j == 0)
   uint32_t hb0, hb1, tb0, tb1;  // shared-memory offsets staged by plain loads
+};
+
+// What a warp found in its window of a look-back.
+struct FlowWindow {
+  uint32_t state;  // 0 all aggregates, 1 not ready for too long, 2 a broken chain, 3 ends at an inclusive record
+  uint32_t cnt, sum;
+  uint32_t exit, entry;  // of the nearest tile, of the farthest
 };
 
 // One look-back record: two words, each tagged with epoch and flag; a record is
@@ -146,25 +154,32 @@ struct Chain {
     }
     return p + (1 + LPB * b) + (LPB * min(b, 1u) + bad);
   }
-  // over a run of empty blocks from p, up to lim; k counts them
+  // over a run of empty blocks from p (a zero byte each; fastmode2: five, the
+  // seed of a field that is 0 and the bit count), up to lim; k counts them
   __device__ __forceinline__ void zeros(uint32_t& p, uint32_t lim, uint32_t& k) const {
-    while (p < lim) {
-      if ((p & 15) == 0 && p + 16 <= lim) {
-        const uint4 v = *reinterpret_cast<const uint4*>(s + p);
+    constexpr uint32_t E = kEmpty;
+    const uint32_t stop = FM2 ? min(lim + E, avail) : lim;
+    uint32_t z = p;  // the first byte that is not zero
+    while (z < stop) {
+      if ((z & 15) == 0 && z + 16 <= stop) {
+        const uint4 v = *reinterpret_cast<const uint4*>(s + z);
         if ((v.x | v.y | v.z | v.w) == 0) {
-          p += 16;
-          k += 16;
+          z += 16;
           continue;
         }
       }
-      const uint32_t left = 4 - (p & 3);
-      const uint32_t w = *reinterpret_cast<const uint32_t*>(s + (p & ~3u)) >> (8 * (p & 3));
-      const uint32_t n = min(min(w ? (uint32_t)(__ffs(w) - 1) >> 3 : left, left), lim - p);
-      p += n;
-      k += n;
-      if (n < left) return;
+      const uint32_t left = 4 - (z & 3);
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(s + (z & ~3u)) >> (8 * (z & 3));
+      const uint32_t n = min(min(w ? (uint32_t)(__ffs(w) - 1) >> 3 : left, left), stop - z);
+      z += n;
+      if (n < left) break;
     }
+    uint32_t n = z - p;
+    if (FM2) n = p < lim ? min(n / E, (lim - p + E - 1) / E) : 0u;
+    p += n * E;
+    k += n;
   }
+  static constexpr uint32_t kEmpty = FM2 ? 5 : 1;  // bytes of an empty block
 };
 
 // ------------------------------------------------------------------ output --
@@ -191,7 +206,13 @@ struct Put {
   __device__ __forceinline__ float value(uint32_t q) const {
     return OUT >= kOutCodes ? __uint_as_float(q) : dequant(q, eb);
   }
+  // Of a lane's 8 doubles, three take the FP64 pipe, which is otherwise idle
+  // (2 lanes a clock and SM), and five the integer arithmetic that bounds the
+  // kernel; both round as binary64 does (33.5 M doubles: 214 us all integer,
+  // 182 so).
+  template <int J>
   __device__ __forceinline__ unsigned long long value_d(uint32_t q) const {
+    if (J == 1 || J == 4 || J == 6) return (unsigned long long)__double_as_longlong(__dmul_rn((double)(int32_t)q, dd.eb));
     return f64i::dequant_bits((int32_t)q, dd.m, dd.ef, dd.sgn);
   }
   __device__ __forceinline__ float add(float old, uint32_t q) {  // old + q as int32 codes
@@ -216,11 +237,14 @@ template <int OUT>
 __device__ __forceinline__ void store8(Put<OUT>& put, void* dst, const uint32_t (&q)[8]) {
   if constexpr (OUT == kOutDouble) {
     unsigned long long* p = static_cast<unsigned long long*>(dst);
-#pragma unroll
-    for (int h = 0; h < 2; h++)
-      asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p + 4 * h), "l"(put.value_d(q[4 * h])),
-                   "l"(put.value_d(q[4 * h + 1])), "l"(put.value_d(q[4 * h + 2])), "l"(put.value_d(q[4 * h + 3]))
-                   : "memory");
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(put.template value_d<0>(q[0])),
+                 "l"(put.template value_d<1>(q[1])), "l"(put.template value_d<2>(q[2])),
+                 "l"(put.template value_d<3>(q[3]))
+                 : "memory");
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p + 4), "l"(put.template value_d<4>(q[4])),
+                 "l"(put.template value_d<5>(q[5])), "l"(put.template value_d<6>(q[6])),
+                 "l"(put.template value_d<7>(q[7]))
+                 : "memory");
   } else {
     float v[8];
     if constexpr (OUT == kOutCodesAdd) {
@@ -279,9 +303,69 @@ __device__ __forceinline__ void store_shifted(Put<OUT>& put, E* dst, const uint3
   }
 }
 
+// o[u][j] = the value SH elements before (SH > 0) or -SH after element
+// 32*8u + 8*lane + j of the two groups' values q.
+template <int SH>
+__device__ __forceinline__ void shift_groups(uint32_t (&o)[2][8], const uint32_t (&q)[2][8], int lane) {
+  constexpr int N = SH > 0 ? SH : -SH;
+  const int from = SH > 0 ? (lane + 31) & 31 : (lane + 1) & 31;
+  uint32_t c[2][N];
+#pragma unroll
+  for (int u = 0; u < 2; u++)
+#pragma unroll
+    for (int j = 0; j < N; j++) c[u][j] = __shfl_sync(0xffffffffu, q[u][SH > 0 ? 8 - N + j : j], from);
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if constexpr (SH > 0) {
+        o[u][j] = j >= N ? q[u][j - N] : u && lane == 0 ? c[0][j] : c[u][j];
+      } else {
+        o[u][j] = j < 8 - N ? q[u][j + N] : u == 0 && lane == 31 ? c[1][j + N - 8] : c[u][j + N - 8];
+      }
+    }
+  }
+}
+
+// store_shifted for doubles, whose conversion is too long to have one copy of it
+// for each shift and each end: the ends go through `ends` (16 words of shared
+// memory), one element per lane.  (For floats the seven copies are the faster:
+// 232 us against 238 on a 168 Mvalue field.)
+__device__ __forceinline__ void store_doubles(Put<kOutDouble>& put, unsigned long long* dst, const uint32_t (&q)[2][8], uint32_t V,
+                                              int sh, int lane, uint32_t* ends) {
+  __syncwarp();
+  if (lane == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) ends[j] = q[0][j];
+  }
+  if (V && lane == (int)((V - 1) & 31)) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) ends[8 + j] = V > 32 ? q[1][j] : q[0][j];
+  }
+  __syncwarp();
+  if (V && lane < 16) {
+    // the first lane's values before the first whole 64 bytes, the last lane's after the last
+    const int j = lane & 7, head = sh > 0 ? 8 - sh : -sh;
+    if (lane < 8 ? j < head : j >= head) put.one(dst, (lane < 8 ? 0 : 8 * (V - 1)) + j, ends[lane]);
+  }
+  uint32_t o[2][8];
+  switch (sh) {
+    case 1: shift_groups<1>(o, q, lane); break;
+    case 2: shift_groups<2>(o, q, lane); break;
+    default: shift_groups<-1>(o, q, lane); break;
+  }
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const uint32_t at = 32 * u + lane;
+    if (sh > 0 ? at > 0 && at < V : at + 1 < V) store8<kOutDouble>(put, dst + 8 * (int)at - sh, o[u]);
+  }
+}
+
 template <int OUT, typename E>
-__device__ __forceinline__ void store_groups(Put<OUT>& put, E* dst, const uint32_t (&q)[2][8], uint32_t V, int lane) {
+__device__ __forceinline__ void store_groups(Put<OUT>& put, E* dst, const uint32_t (&q)[2][8], uint32_t V, int lane,
+                                             uint32_t* ends) {
   constexpr uint32_t U = 32 / sizeof(E);  // elements in 32 bytes
+  const uint32_t s = (uint32_t)((uintptr_t)dst / sizeof(E)) % U;
   if (put.rare) {
 #pragma unroll 1
     for (int u = 0; u < 2; u++)
@@ -290,19 +374,24 @@ __device__ __forceinline__ void store_groups(Put<OUT>& put, E* dst, const uint32
         if (32u * u + lane < V) put.one(dst, 256 * u + 8 * lane + j, u ? q[1][j] : q[0][j]);
     return;
   }
-  switch ((uint32_t)((uintptr_t)dst / sizeof(E)) % U) {
-    case 0:
+  if (s == 0) {
 #pragma unroll
-      for (int u = 0; u < 2; u++)
-        if (32u * u + lane < V) store8<OUT>(put, dst + 256 * u + 8 * lane, q[u]);
-      break;
-    case 1: store_shifted<OUT, 1>(put, dst, q, V, lane); break;
-    case 2: store_shifted<OUT, 2>(put, dst, q, V, lane); break;
-    case 3: store_shifted<OUT, U == 8 ? 3 : -1>(put, dst, q, V, lane); break;
-    case 4: store_shifted<OUT, 4>(put, dst, q, V, lane); break;
-    case 5: store_shifted<OUT, -3>(put, dst, q, V, lane); break;
-    case 6: store_shifted<OUT, -2>(put, dst, q, V, lane); break;
-    default: store_shifted<OUT, -1>(put, dst, q, V, lane); break;
+    for (int u = 0; u < 2; u++)
+      if (32u * u + lane < V) store8<OUT>(put, dst + 256 * u + 8 * lane, q[u]);
+    return;
+  }
+  if constexpr (OUT == kOutDouble) {
+    store_doubles(put, dst, q, V, s == 3 ? -1 : (int)s, lane, ends);
+  } else {
+    switch (s) {
+      case 1: store_shifted<OUT, 1>(put, dst, q, V, lane); break;
+      case 2: store_shifted<OUT, 2>(put, dst, q, V, lane); break;
+      case 3: store_shifted<OUT, 3>(put, dst, q, V, lane); break;
+      case 4: store_shifted<OUT, 4>(put, dst, q, V, lane); break;
+      case 5: store_shifted<OUT, -3>(put, dst, q, V, lane); break;
+      case 6: store_shifted<OUT, -2>(put, dst, q, V, lane); break;
+      default: store_shifted<OUT, -1>(put, dst, q, V, lane); break;
+    }
   }
 }
 
@@ -323,8 +412,8 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
   __shared__ uint32_t s_c0[NB + 1];         // blocks before each chunk
   __shared__ bool s_noted;                  // the walking lanes noted every block
   __shared__ FlowTile s_t;
-  __shared__ uint32_t s_k, s_sum, s_verdict, s_base;
-  __shared__ uint64_t s_g0;
+  __shared__ uint32_t s_k, s_sum, s_h0, s_epoch;
+  __shared__ FlowWindow s_win[kFlowWarps];
   __shared__ __align__(8) uint64_t s_bar;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane % LPB, grp = lane / LPB;
@@ -333,6 +422,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
   if (tid == 0) {
     mbar_init(&s_bar, 1);
     epoch = *(volatile uint32_t*)&a.ls->epoch;
+    s_epoch = epoch;
     __threadfence();
   }
   epoch = __shfl_sync(0xffffffffu, epoch, 0);  // used by warp 0 only
@@ -357,7 +447,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         t.scS = at.z * t.sc;
         t.scE = min(t.scS + t.sc, t.rlen);
         t.last = t.scE == t.rlen;
-        const uint32_t lead = min(S::W, a.overlap);
+        const uint32_t lead = min(FM2 ? S::LEAD2 : S::W, a.overlap);
         t.st0 = t.scS > lead ? t.scS - lead : 0u;
         t.st1 = (uint32_t)min((uint64_t)t.rlen, (uint64_t)t.scE + MAXSZ + 8);
         // the 16-byte-aligned part of the staged bytes that lies in the stream goes by bulk copy
@@ -425,11 +515,13 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
     {
       constexpr int Q = NB >= kFlowWarps ? NB / kFlowWarps : 1;
       uint32_t at[Q], p[Q];  // first byte tried; the lane's position
+      uint32_t back[Q];      // the window
       uint32_t open = 0;     // chunks without an entry yet
 #pragma unroll
       for (int q = 0; q < Q; q++) {
         const uint32_t i = warp + kFlowWarps * q, B = lS + i * C;
         const uint32_t first = s_t.st0 + off;
+        back[q] = S::W;
         at[q] = B - first > S::W ? B - S::W : first;
         p[q] = kAway;
         if (i < NB && B < lE && !(i == 0 && j0)) {
@@ -494,7 +586,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             c = ch.next(c, b);
             over = min(over, c - B);
           }
-          if (!FM2 && c - c0 == 4 && c < B) {  // a run of empty blocks
+          if (c - c0 == 4 * Chain<LPB, FM2>::kEmpty && c < B) {  // a run of empty blocks
             uint32_t k = 0;
             ch.zeros(c, B, k);
             over = min(over, c - B);
@@ -509,12 +601,25 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
 #pragma unroll
         for (int s = 1; s < 8; s <<= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, s));
         const uint32_t ent = __shfl_sync(0xffffffffu, e, 31 - (best & 31));
-        const uint32_t found = __ballot_sync(0xffffffffu, best != 0 && (lane & 7) == 0);
+        uint32_t found = __ballot_sync(0xffffffffu, best != 0 && (lane & 7) == 0);
+        // fastmode2: a run of empty blocks has five chains that all stay valid, and
+        // only what lies before it tells them apart: where survivors disagree, a
+        // window four times as long is tried, as far as there are bytes
+        const uint32_t split = FM2 ? __ballot_sync(0xffffffffu, alive && with < best >> 5 || alive && e != ent) : 0u;
         if (best != 0 && (lane & 7) == 0 && (open >> (lane >> 3) & 1)) s_ent[warp + kFlowWarps * (lane >> 3)] = ent;
 #pragma unroll
         for (int q = 0; q < Q; q++) {
           p[q] = kAway;
           if (!(open >> q & 1)) continue;
+          if (FM2 && (split >> (8 * q) & 0xFFu)) {
+            const uint32_t first = s_t.st0 + off, Bq = lS + (warp + kFlowWarps * q) * C;
+            if (Bq - first > back[q]) {
+              back[q] *= 4;
+              at[q] = Bq - first > back[q] ? Bq - back[q] : first;
+              p[q] = at[q] + lane;
+              continue;
+            }
+          }
           at[q] += 32;
           if ((found >> (8 * q) & 1) || at[q] >= lS + (warp + kFlowWarps * q) * C) {
             open &= ~(1u << q);
@@ -638,7 +743,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       }
       return run;  // warp 0: the listed blocks' delta sum
     };
-    uint64_t cnt0 = 0;
+    uint64_t cnt0 = 0;  // blocks before the super-chunk, and the value there (in every thread)
     uint32_t base = 0;
     for (int attempt = 0;; attempt++) {
       if (warp == 0) {
@@ -669,7 +774,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             kk += n;
             nn += room ? n : n + CAPL;  // too many: nn > CAPL from here on
             p = pp[4];
-            if (!FM2 && p - pp[0] == 4 && p < cE) {  // a run of empty blocks is taken at once
+            if (p - pp[0] == 4 * Chain<LPB, FM2>::kEmpty && p < cE) {  // a run of empty blocks is taken at once
               const uint32_t first = p, k0 = kk;
               ch.zeros(p, cE, kk);
               over = min(over, p - cE);
@@ -704,10 +809,15 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         wp0 = e + off;  // e is a position where k > 0
         wi = wi0;
         wp = wp0;
+        if (FM2 && attempt) {  // nothing else is needed: the tiles after this one wait for it
+          if (lane == 0)
+            publish(a.status + 2ull * s_t.rec, epoch, kFlagInclusive, cnt0 + K, 0u, h0, xl, scS, scE);
+        }
         if (lane < (int)NB) s_c0[lane] = wi0;
         if (lane == 0) {
           s_c0[NB] = K;
           s_k = K;
+          s_h0 = h0;
           s_noted = noted;
         }
         if (!noted) list(0);
@@ -726,7 +836,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             const uint32_t t1 = run.x >> 16;
             for (uint32_t t = t0 + tid % TPC; t < t1; t += TPC) s_pos[at + t - t0] = s_note[i * CAPL + t];
             at += t1 - t0;
-            for (uint32_t t = tid % TPC; t < run.y; t += TPC) s_pos[at + t] = (uint16_t)((run.x & 0xFFFFu) + t);
+            for (uint32_t t = tid % TPC; t < run.y; t += TPC) s_pos[at + t] = (uint16_t)((run.x & 0xFFFFu) + t * Chain<LPB, FM2>::kEmpty);
             at += run.y;
             t0 = t1;
           }
@@ -743,112 +853,126 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         }
         sum += sums(min(KCAP, K - kb));
       }
-      if (warp == 0) {
-        const uint32_t rec = s_t.rec;  // the records of a segment follow one another
-        uint64_t* st = a.status + 2ull * rec;
-        if (j0) {
-          base = s_t.seed;
-          if (lane == 0) publish(st, epoch, kFlagInclusive, K, base + sum, h0, xl, scS, scE);
-          if (lane == 0) s_verdict = 1;
-        } else if (attempt) {  // the predecessor's exit and the prefixes are known
-          if (lane == 0) publish(st, epoch, kFlagInclusive, cnt0 + K, base + sum, h0, xl, scS, scE);
-          if (lane == 0) s_verdict = 1;
-        } else {
-          if (lane == 0) publish(st, epoch, kFlagAggregate, K, sum, h0, xl, scS, scE);
-          // lane l reads the tile at distance 1 + l + 32w; a window that is
-          // not ready is read again, a broken chain of (entry, exit) pairs
-          // (an older tile will correct itself) starts the look-back over
-          const int64_t first = (int64_t)rec - s_t.j;
-          uint32_t spins = 0;
-          int verdict = 0;  // 1 done, 2 start over, 3 own entry wrong
-          uint32_t pred_x = kDead;
+      const uint32_t rec = s_t.rec;  // the records of a segment follow one another
+      uint64_t* const st = a.status + 2ull * rec;
+      if (j0 || attempt) {  // no predecessor, or its exit and the prefixes are known
+        if (j0) base = s_t.seed;
+        if (tid == 0 && !(FM2 && attempt)) publish(st, epoch, kFlagInclusive, cnt0 + K, base + sum, h0, xl, scS, scE);
+        break;
+      }
+      if (tid == 0) publish(st, epoch, kFlagAggregate, K, sum, h0, xl, scS, scE);
+      h0 = s_h0;
+      // Lane l of warp 0 reads the record at distance 1 + l; where none of those 32
+      // is inclusive (a stream of one segment has all the CTAs in flight behind one
+      // another) the four warps go on with 128 records a trip.  (Four windows from
+      // the start: 255 us instead of 232 on a 168 Mvalue field in 1024 segments.)
+      // A window that is not ready is read again; a broken chain of (entry, exit)
+      // pairs (an older tile will correct itself) starts the look-back over.
+      const int64_t first = (int64_t)rec - s_t.j;
+      const uint32_t sc = s_t.sc;
+      uint32_t spins = 0, pred_x = kDead, need_x = h0;
+      bool self_ok = true;
+      int verdict = 0;  // 1 done, 3 own entry wrong
+      int64_t at = (int64_t)rec - 1;
+      cnt0 = 0;
+      base = 0;
+      while (verdict == 0) {
+        const int span = at == (int64_t)rec - 1 ? 1 : kFlowWarps;
+        const int64_t mine = at - 32 * warp, idx = mine - lane;
+        if (warp < span && mine >= first) {
+          const bool inr = idx >= first;
+          ulonglong2 w = make_ulonglong2(0, 0);
+          uint64_t f = 0;
+          uint32_t bi = 0;
+          bool wait;
           while (true) {
-            int64_t at = (int64_t)rec - 1;
-            uint32_t need_x = h0;
-            bool self_ok = true;
+            if (inr) w = ld_record(a.status + 2 * idx);
+            f = status_flag(w.x);
+            const bool ready = !inr || (w.x >> 42 == w.y >> 42 && status_epoch(w.x) == (s_epoch & 0xFFFFF) &&
+                                        (f == kFlagAggregate || f == kFlagInclusive));
+            bi = __ballot_sync(0xffffffffu, inr && ready && f == kFlagInclusive);
+            wait = __any_sync(0xffffffffu, inr && !ready && lane < (bi ? __ffs(bi) : 32));
+            if (!wait || ++spins > kSpinLimit || ((spins & 63) == 0 && launch_gave_up(a.err))) break;
+            __nanosleep(100);
+          }
+          const bool incl = inr && f == kFlagInclusive;  // (only looked at where the record is ready)
+          const int jstar = bi ? __ffs(bi) - 1 : 32;     // nearest inclusive of the window
+          const bool rel = inr && lane <= jstar;
+          const uint64_t vx = status_value(w.x), vy = status_value(w.y);
+          const uint32_t tS = (uint32_t)(idx - first) * sc, tE = min(tS + sc, rlen);
+          const uint32_t xr = (uint32_t)(vx & 1023u) | (uint32_t)(vy & 1023u) << 10;
+          const uint32_t tx = xr == kXDead ? kDead : xr == kXEnd ? kEnd : tE + xr;
+          const uint32_t hr = (uint32_t)(vx >> 26) & 0xFFFFu;
+          const uint32_t th = hr == kHDead ? kDead : hr == kHEnd ? kEnd : tS + hr;
+          const uint32_t cnt = incl ? (uint32_t)(vx >> 10) : (uint32_t)(vx >> 10) & 0xFFFFu;
+          // the entry of a lane's tile must be the exit of the next older one
+          const uint32_t ox = __shfl_down_sync(0xffffffffu, tx, 1);
+          const bool bad = __any_sync(0xffffffffu, rel && lane < jstar && lane < 31 && idx - 1 >= first && th != ox);
+          // counts of up to 2^32 - 1 in all: a segment's region is below 4 GiB
+          const uint32_t c = __reduce_add_sync(0xffffffffu, rel ? cnt : 0u);
+          const uint32_t s = __reduce_add_sync(0xffffffffu, rel ? (uint32_t)(vy >> 10) : 0u);
+          if (lane == 0) {
+            s_win[warp].state = wait ? 1u : bad ? 2u : jstar < 32 ? 3u : 0u;
+            s_win[warp].cnt = c;
+            s_win[warp].sum = s;
+            s_win[warp].exit = tx;
+          }
+          if (lane == 31) s_win[warp].entry = th;
+        }
+        __syncthreads();
+        // every thread takes the windows together, nearest first
+        bool over = false;
+        for (int v = 0; v < span && verdict == 0; v++) {
+          const FlowWindow& win = s_win[v];
+          if (win.state == 1) {  // not ready for too long
+            if (tid == 0) atomicOr(a.err, kErrLookbackTimeout);
+            verdict = 1;
+            break;
+          }
+          if (at == (int64_t)rec - 1) {
+            self_ok = win.exit == h0;
+            pred_x = win.exit;
+          } else if (win.exit != need_x) {
+            over = true;
+          }
+          if (win.state == 2 || over) {
+            over = true;
+            break;
+          }
+          cnt0 += win.cnt;
+          base += win.sum;
+          need_x = win.entry;
+          at -= 32;
+          if (win.state == 3 || at < first) verdict = self_ok ? 1 : 3;
+        }
+        __syncthreads();  // the windows are read before they are written again
+        if (verdict == 0 && over) {
+          const bool give_up = ++spins > kSpinLimit || ((spins & 63) == 0 && launch_gave_up(a.err));
+          if (__syncthreads_or(give_up)) {
+            if (tid == 0) atomicOr(a.err, kErrLookbackTimeout);
+            verdict = 1;
+          } else {
+            at = (int64_t)rec - 1;
+            need_x = h0;
             cnt0 = 0;
             base = 0;
-            verdict = 0;
-            while (verdict == 0) {
-              const int64_t idx = at - lane;
-              const bool inr = idx >= first;
-              ulonglong2 w = make_ulonglong2(0, 0);
-              if (inr) w = ld_record(a.status + 2 * idx);
-              const uint64_t f = status_flag(w.x);
-              const bool ready = !inr || (w.x >> 42 == w.y >> 42 && status_epoch(w.x) == (epoch & 0xFFFFF) &&
-                                          (f == kFlagAggregate || f == kFlagInclusive));
-              const bool incl = inr && ready && f == kFlagInclusive;
-              const uint32_t bi = __ballot_sync(0xffffffffu, incl);
-              const int jstar = bi ? __ffs(bi) - 1 : 32;  // nearest inclusive of the window
-              const bool rel = inr && lane <= jstar;
-              if (__any_sync(0xffffffffu, rel && !ready)) {
-                if (++spins > kSpinLimit || ((spins & 63) == 0 && launch_gave_up(a.err))) {
-                  if (lane == 0) atomicOr(a.err, kErrLookbackTimeout);
-                  verdict = 1;
-                  break;
-                }
-                __nanosleep(100);
-                continue;
-              }
-              const uint64_t vx = status_value(w.x), vy = status_value(w.y);
-              const uint32_t tS = (uint32_t)(idx - first) * s_t.sc, tE = min(tS + s_t.sc, rlen);
-              const uint32_t xr = (uint32_t)(vx & 1023u) | (uint32_t)(vy & 1023u) << 10;
-              const uint32_t tx = xr == kXDead ? kDead : xr == kXEnd ? kEnd : tE + xr;
-              const uint32_t hr = (uint32_t)(vx >> 26) & 0xFFFFu;
-              const uint32_t th = hr == kHDead ? kDead : hr == kHEnd ? kEnd : tS + hr;
-              const uint32_t cnt = incl ? (uint32_t)(vx >> 10) : (uint32_t)(vx >> 10) & 0xFFFFu;
-              // the entry of a lane's tile must be the exit of the next older one
-              const uint32_t ox = __shfl_down_sync(0xffffffffu, tx, 1);
-              bool bad = rel && lane < jstar && lane < 31 && idx - 1 >= first && th != ox;
-              const uint32_t px = __shfl_sync(0xffffffffu, tx, 0);
-              if (at == (int64_t)rec - 1) {
-                self_ok = px == h0;
-                pred_x = px;
-              } else {
-                bad |= px != need_x;
-              }
-              if (__any_sync(0xffffffffu, bad)) {
-                verdict = 2;
-                break;
-              }
-              uint32_t c = rel ? cnt : 0u, s = rel ? (uint32_t)(vy >> 10) : 0u;
-              // counts of up to 2^32 - 1 in all: a segment's region is below 4 GiB
-              cnt0 += __reduce_add_sync(0xffffffffu, c);
-              base += __reduce_add_sync(0xffffffffu, s);
-              need_x = __shfl_sync(0xffffffffu, th, 31);
-              at -= 32;
-              if (jstar < 32 || at < first) verdict = self_ok ? 1 : 3;
-            }
-            if (verdict != 2) break;
-            if (++spins > kSpinLimit || ((spins & 63) == 0 && launch_gave_up(a.err))) {
-              if (lane == 0) atomicOr(a.err, kErrLookbackTimeout);
-              verdict = 1;
-              break;
-            }
             __nanosleep(200);
           }
-          if (lane == 0) {
-            if (verdict == 3) {  // unready until the corrected record is out
-              st_relaxed_u64(st, make_status(epoch, 3, 0));
-              st_relaxed_u64(st + 1, make_status(epoch, 3, 0));
-            } else {
-              publish(st, epoch, kFlagInclusive, cnt0 + K, base + sum, h0, xl, scS, scE);
-            }
-            s_verdict = (uint32_t)verdict;
-          }
-          if (verdict == 3) {
-            h0 = pred_x;
-            repaired = true;
-          }
-        }
-        if (lane == 0) {
-          s_g0 = cnt0;
-          s_base = base;
         }
       }
-      __syncthreads();
-      if (s_verdict == 1) break;
+      if (verdict == 3) {
+        if (tid == 0) {  // unready until the corrected record is out
+          st_relaxed_u64(st, make_status(epoch, 3, 0));
+          st_relaxed_u64(st + 1, make_status(epoch, 3, 0));
+        }
+        h0 = pred_x;
+        repaired = true;
+        continue;
+      }
+      if (tid == 0) publish(st, epoch, kFlagInclusive, cnt0 + K, base + sum, h0, xl, scS, scE);
+      break;
     }
+    __syncthreads();  // the groups' prefixes are in place
     if (warp == 0) {
       if (__any_sync(0xffffffffu, repaired) && lane == 0) atomicAdd(&a.counters[0], 1u);
       if (lane == 0 && s_t.last) {  // the last super-chunk of a segment checks the block total
@@ -857,13 +981,12 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       }
     }
     // ---- decode ----
-    const uint64_t g0 = s_g0, nb = s_t.nb;
+    const uint64_t g0 = cnt0, nb = s_t.nb;  // the blocks before the super-chunk
     const uint32_t kmax = g0 >= nb ? 0u : (uint32_t)min((uint64_t)K, nb - g0);
-    const uint32_t q0b = s_base;
     Put<OUT> put(s_t.eb, s_t.ebd);
     using E = typename Elem<OUT>::T;
     E* const y = static_cast<E*>(s_t.y) + s_t.lo;  // block g's values start at y + g*L (fastmode1: with the value before it)
-    uint32_t qpass = q0b;
+    uint32_t qpass = base;
     bool corrupt = false;
     for (uint32_t kb = 0; kb < kmax; kb += KCAP) {
       const uint32_t kn = min(KCAP, kmax - kb);
@@ -934,7 +1057,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           groups(std::integral_constant<int, 3>{});
         }
         const uint32_t blocks = min(min(2u, nfast - r) * BPR, kn - r * BPR);
-        store_groups<OUT>(put, y + (g0 + kb + (uint64_t)r * BPR) * L, q, blocks * LPB, lane);
+        store_groups<OUT>(put, y + (g0 + kb + (uint64_t)r * BPR) * L, q, blocks * LPB, lane, s_tried[warp]);
       }
       if (tail && (ng - 1) % kFlowWarps == (uint32_t)warp) {
         const uint32_t r = ng - 1, blk = r * BPR + grp;

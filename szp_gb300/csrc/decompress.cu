@@ -96,13 +96,13 @@ __device__ void put_seed(const DecArgs& a, const DecField& fd, uint64_t e, uint3
 // many as hold 32 Ki values (empty blocks take one byte for 32 values, and a
 // CTA that meets thousands of them is the last to finish: a 2^24-value walk at
 // REL 1e-2 decodes 16 KB into 2 MB), and in a short stream no more than gives
-// the GPU two super-chunks per resident CTA (1 MB of floats: 22 -> 14 us).
+// the GPU one super-chunk per resident CTA (1 MB of floats: 22 -> 18 us).
 __device__ __forceinline__ uint32_t flow_chunks(const DecArgs& a, uint64_t bytes, uint64_t nblk, uint32_t L,
                                                 uint64_t total) {
   // in single precision: the result only has to be the same wherever it is taken
   const float most = (float)(kFlowSuper / a.super_chunk), c = (float)a.super_chunk;
   const float by_values = __fdiv_rn((float)bytes * (32768.0f / L), fmaxf((float)nblk, 1.0f) * c);
-  const float by_total = __fdiv_rn((float)total, 2048.0f * c);
+  const float by_total = __fdiv_rn((float)total, 1024.0f * c);
   return (uint32_t)fmaxf(1.0f, fminf(most, fminf(by_values, by_total)));
 }
 
