@@ -115,11 +115,13 @@ struct FlowWindow {
 // with the exit counted from the super-chunk's end.
 constexpr uint32_t kHDead = 0xFFFFu, kHEnd = 0xFFFEu, kXDead = 0xFFFu, kXEnd = 0xFFEu;
 
+// an aggregate for a super-chunk's second entry (a tag of its own, so that no read record mixes two)
+constexpr uint64_t kFlagSecond = 0;
 __device__ __forceinline__ void publish(uint64_t* st, uint32_t epoch, uint64_t flag, uint64_t cnt, uint32_t sum,
                                         uint32_t h, uint32_t x, uint32_t scS, uint32_t scE) {
   const uint32_t xr = x == kDead ? kXDead : x == kEnd ? kXEnd : x - scE;
   const uint32_t hr = h == kDead ? kHDead : h == kEnd ? kHEnd : h - scS;
-  const uint64_t head = flag == kFlagAggregate ? ((uint64_t)hr << 16 | cnt) : cnt;
+  const uint64_t head = flag != kFlagInclusive ? ((uint64_t)hr << 16 | cnt) : cnt;
   st_relaxed_u64(st, make_status(epoch, flag, head << 10 | (xr & 1023u)));
   st_relaxed_u64(st + 1, make_status(epoch, flag, (uint64_t)sum << 10 | (xr >> 10)));
 }
@@ -745,7 +747,9 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
     };
     uint64_t cnt0 = 0;  // blocks before the super-chunk, and the value there (in every thread)
     uint32_t base = 0;
-    for (int attempt = 0;; attempt++) {
+    bool known = j0;  // the entry is the true one, and cnt0 and base are known
+    uint64_t kind = kFlagAggregate;
+    while (true) {
       if (warp == 0) {
         uint32_t e = lane == 0 ? h0 : e0, k = 0, x = kDead;
         bool need = act, noted = true;
@@ -809,7 +813,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         wp0 = e + off;  // e is a position where k > 0
         wi = wi0;
         wp = wp0;
-        if (FM2 && attempt) {  // nothing else is needed: the tiles after this one wait for it
+        if (FM2 && known && !j0) {  // nothing else is needed: the tiles after this one wait for it
           if (lane == 0)
             publish(a.status + 2ull * s_t.rec, epoch, kFlagInclusive, cnt0 + K, 0u, h0, xl, scS, scE);
         }
@@ -855,24 +859,32 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       }
       const uint32_t rec = s_t.rec;  // the records of a segment follow one another
       uint64_t* const st = a.status + 2ull * rec;
-      if (j0 || attempt) {  // no predecessor, or its exit and the prefixes are known
+      if (known) {
         if (j0) base = s_t.seed;
-        if (tid == 0 && !(FM2 && attempt)) publish(st, epoch, kFlagInclusive, cnt0 + K, base + sum, h0, xl, scS, scE);
+        if (tid == 0 && (!FM2 || j0)) publish(st, epoch, kFlagInclusive, cnt0 + K, base + sum, h0, xl, scS, scE);
         break;
       }
-      if (tid == 0) publish(st, epoch, kFlagAggregate, K, sum, h0, xl, scS, scE);
+      if (tid == 0) publish(st, epoch, kind, K, sum, h0, xl, scS, scE);
       h0 = s_h0;
       // Lane l of warp 0 reads the record at distance 1 + l; where none of those 32
       // is inclusive (a stream of one segment has all the CTAs in flight behind one
       // another) the four warps go on with 128 records a trip.  (Four windows from
       // the start: 255 us instead of 232 on a 168 Mvalue field in 1024 segments.)
       // A window that is not ready is read again; a broken chain of (entry, exit)
-      // pairs (an older tile will correct itself) starts the look-back over.
+      // pairs (an older tile will correct itself) starts the look-back over.  A
+      // tile whose entry is not its neighbour's exit walks again at once, from that
+      // exit (if it is one: no tile gives up an entry for a walk that went wrong),
+      // and publishes a second aggregate, so that the wrong entries of a segment
+      // are mended side by side and not each after the prefixes of the one before
+      // (2 M values of one segment whose entries are often wrong: 123 -> 85 us;
+      // the 168 Mvalue field 233 -> 225).  When that was not the true entry either,
+      // the next walk waits until the whole chain is known.
       const int64_t first = (int64_t)rec - s_t.j;
       const uint32_t sc = s_t.sc;
+      const bool may_second = (s_epoch & 0xFFFFF) != 0;  // a zeroed word must not read as a second claim
       uint32_t spins = 0, pred_x = kDead, need_x = h0;
       bool self_ok = true;
-      int verdict = 0;  // 1 done, 3 own entry wrong
+      int verdict = 0;  // 1 done, 2 entry unlike the neighbour's exit, 3 own entry wrong
       int64_t at = (int64_t)rec - 1;
       cnt0 = 0;
       base = 0;
@@ -889,7 +901,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             if (inr) w = ld_record(a.status + 2 * idx);
             f = status_flag(w.x);
             const bool ready = !inr || (w.x >> 42 == w.y >> 42 && status_epoch(w.x) == (s_epoch & 0xFFFFF) &&
-                                        (f == kFlagAggregate || f == kFlagInclusive));
+                                        (f == kFlagAggregate || f == kFlagInclusive || f == kFlagSecond && may_second));
             bi = __ballot_sync(0xffffffffu, inr && ready && f == kFlagInclusive);
             wait = __any_sync(0xffffffffu, inr && !ready && lane < (bi ? __ffs(bi) : 32));
             if (!wait || ++spins > kSpinLimit || ((spins & 63) == 0 && launch_gave_up(a.err))) break;
@@ -932,6 +944,10 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           if (at == (int64_t)rec - 1) {
             self_ok = win.exit == h0;
             pred_x = win.exit;
+            if (!self_ok && kind == kFlagAggregate && may_second && pred_x < kEnd) {
+              verdict = 2;
+              break;
+            }
           } else if (win.exit != need_x) {
             over = true;
           }
@@ -960,7 +976,9 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           }
         }
       }
-      if (verdict == 3) {
+      if (verdict >= 2) {
+        known = verdict == 3;
+        kind = kFlagSecond;
         if (tid == 0) {  // unready until the corrected record is out
           st_relaxed_u64(st, make_status(epoch, 3, 0));
           st_relaxed_u64(st + 1, make_status(epoch, 3, 0));
