@@ -96,13 +96,17 @@ __device__ void put_seed(const DecArgs& a, const DecField& fd, uint64_t e, uint3
 // many as hold 32 Ki values (empty blocks take one byte for 32 values, and a
 // CTA that meets thousands of them is the last to finish: a 2^24-value walk at
 // REL 1e-2 decodes 16 KB into 2 MB), and in a short stream no more than gives
-// the GPU one super-chunk per resident CTA (1 MB of floats: 22 -> 18 us).
+// the GPU one super-chunk per resident CTA (1 MB of floats: 22 -> 18 us), or
+// two of the same size where one each is not enough (21.5 MB in one segment as
+// 1312 super-chunks on 1064 CTAs: 208 us a call; as 1955: 162.  At three turns the
+// smaller ones lost 3 %).
 __device__ __forceinline__ uint32_t flow_chunks(const DecArgs& a, uint64_t bytes, uint64_t nblk, uint32_t L,
                                                 uint64_t total) {
   // in single precision: the result only has to be the same wherever it is taken
   const float most = (float)(kFlowSuper / a.super_chunk), c = (float)a.super_chunk;
   const float by_values = __fdiv_rn((float)bytes * (32768.0f / L), fmaxf((float)nblk, 1.0f) * c);
-  const float by_total = __fdiv_rn((float)total, 1024.0f * c);
+  const float share = __fdiv_rn((float)total, 1024.0f * c), turns = ceilf(__fdiv_rn(share, most));
+  const float by_total = turns <= 1.0f ? share : turns <= 2.0f ? ceilf(__fdiv_rn(share, turns)) : most;
   return (uint32_t)fmaxf(1.0f, fminf(most, fminf(by_values, by_total)));
 }
 
