@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
+#include <cstddef>
 #include <cstring>
 #include <atomic>
 #include <memory>
@@ -130,12 +131,12 @@ struct DevBuf {
 // Device scalars of one workspace.
 struct DevMisc {
   LaunchState ls;
-  uint32_t err;
+  uint32_t err;          // err, rel_counter and out_size go to the host in one copy
   uint32_t rel_counter;
   uint64_t out_size;
   float eb;
   float pad;
-  uint32_t verify[4];  // [0] locate repairs of the last launch
+  uint32_t verify[4];  // [0] repairs of the last decode
   double ebd;          // REL bound of float64 data
   double invd;         // and its inverse
 };
@@ -446,13 +447,13 @@ int compress_launch(Workspace& w, const CompressJob& j, cudaStream_t st) {
 // Copies the stream size and error word to pinned memory and waits.
 int finish_sync(Workspace& w, cudaStream_t st, size_t* out_size) {
   DevMisc* dm = w.dm();
-  CU(cudaMemcpyAsync(w.h_small, &dm->out_size, 8, cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(w.h_small + 8, &dm->err, 4, cudaMemcpyDeviceToHost, st));
+  static_assert(offsetof(DevMisc, out_size) == offsetof(DevMisc, err) + 8, "one copy takes both");
+  CU(cudaMemcpyAsync(w.h_small, &dm->err, 16, cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
   uint64_t sz;
   uint32_t err;
-  memcpy(&sz, w.h_small, 8);
-  memcpy(&err, w.h_small + 8, 4);
+  memcpy(&err, w.h_small, 4);
+  memcpy(&sz, w.h_small + 8, 8);
   t_notices = (err & kErrQuantRange) ? 1 : 0;
   if (out_size) *out_size = (size_t)sz;
   return status_from_err(err);
@@ -513,8 +514,7 @@ int decompress_launch(Workspace& w, const DecompressJob& j, cudaStream_t st) {
   }
   const size_t plan_bytes = 64 + 4ull * (j.T + 1) + 16ull * j.T + 64;
   CU(w.plan.ensure(plan_bytes));
-  DevMisc* dm = w.dm();
-  CU(cudaMemsetAsync(&dm->err, 0, sizeof(uint32_t), st));
+  DevMisc* dm = w.dm();  // the setup kernel clears err and verify[0]
 
   DecArgs a;
   memset(&a, 0, sizeof a);
@@ -558,7 +558,6 @@ int decompress_launch(Workspace& w, const DecompressJob& j, cudaStream_t st) {
   } else if (locate_smem_bytes(SC, a.overlap, maxsz) > 200 * 1024) {
     return fail(SZP_GB300_EINVAL, "blockSize too large");
   }
-  CU(cudaMemsetAsync(dm->verify, 0, sizeof(uint32_t), st));
 
   w.mark(kSlotSetup, 0, st);
   CU(launch_dec_setup(a, st));

@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
   __shared__ volatile uint32_t s_stop_k;
   __shared__ volatile uint32_t s_started;
   __shared__ __align__(8) uint64_t s_full[NS], s_aggb[NS], s_packed[NS], s_empty[NS];
+  if (!BATCH) wait_for_previous();
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 36) s_thr[threadIdx.x] = a.thr.thr[threadIdx.x];
@@ -1072,6 +1073,7 @@ __device__ __forceinline__ void rel_finish(const RelArgs& a, float mn, float mx)
 }
 
 __global__ void __launch_bounds__(256) rel_bound_kernel(RelArgs a) {
+  let_next_start();
   float mn = INFINITY, mx = -INFINITY;
   const uint64_t n = a.n;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1118,6 +1120,7 @@ constexpr int kRelStages = 3;
 constexpr uint32_t kRelChunk = 4096;  // floats per bulk copy
 
 __global__ void __launch_bounds__(256) rel_bound_bulk(RelArgs a, uint64_t body0, uint64_t nbody) {
+  let_next_start();
   extern __shared__ __align__(16) float s_stage[];  // kRelStages * kRelChunk floats
   __shared__ __align__(8) uint64_t s_full[kRelStages];
   float mn = INFINITY, mx = -INFINITY;
@@ -1372,6 +1375,7 @@ static cudaError_t launch_lanes(const CompressArgs& a, cudaStream_t st) {
   const uint32_t s_grid = (uint32_t)c;
   const uint32_t grid = a.ntiles < s_grid ? a.ntiles : s_grid;
   if (grid == 0) return cudaSuccess;
+  if (!BATCH) return launch_behind(k, grid, kPipeThreads, smem, st, a, slot);
   k<<<grid, kPipeThreads, smem, st>>>(a, slot);
   return cudaGetLastError();
 }
@@ -1554,6 +1558,7 @@ cudaError_t launch_rel_bound_f64(const RelArgs& a, uint32_t grid, cudaStream_t s
 __global__ void __launch_bounds__(256) quantize_f64_kernel(const double* __restrict__ x, int32_t* __restrict__ q,
                                                            uint64_t n, double invd, const double* invd_dev,
                                                            uint32_t* err) {
+  let_next_start();
   const f64i::Inverse io = f64i::prepare_inverse(f64i::bits_of(invd_dev ? *invd_dev : invd));
   bool bad = false;
   const uint64_t h = min(n, (uint64_t)((((uintptr_t)x & 15) >> 3)));

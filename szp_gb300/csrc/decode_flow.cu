@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
   __shared__ uint32_t s_k, s_sum, s_h0, s_epoch;
   __shared__ FlowWindow s_win[kFlowWarps];
   __shared__ __align__(8) uint64_t s_bar;
+  if (!BATCH) wait_for_previous();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane % LPB, grp = lane / LPB;
   uint32_t epoch = 0;
@@ -1166,6 +1167,7 @@ cudaError_t launch_one(const DecArgs& a, cudaStream_t st) {
   const uint32_t cap = (uint32_t)c;
   const uint32_t grid = a.nlocate_ctas < cap ? a.nlocate_ctas : cap;
   if (grid == 0) return cudaSuccess;
+  if (!BATCH) return launch_behind(k, grid, kFlowThreads, smem, st, a);
   k<<<grid, kFlowThreads, smem, st>>>(a);
   return cudaGetLastError();
 }

@@ -121,6 +121,13 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   __shared__ uint32_t s_cb[kTurnT + 1], s_k[kTurnT];  // tickets before each segment; its chunks per super-chunk
   __shared__ uint32_t s_bad, s_base0, s_all, s_most;  // s_most: of the segment with the most super-chunks
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  if (!BATCH) {
+    let_next_start();
+    if (threadIdx.x == 0) {  // (a batch clears its fields' status in a launch before)
+      *a.err = 0;
+      a.counters[0] = 0;
+    }
+  }
   uint64_t len = fd.len;
   if (fd.len_dev) {
     uint64_t l2 = *fd.len_dev;

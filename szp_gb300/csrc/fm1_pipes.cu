@@ -443,6 +443,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
   __shared__ volatile uint32_t s_stop_k;    // the producer's stop position
   __shared__ volatile uint32_t s_cstop_k;   // the compute warps' stop position (for the control warp)
   __shared__ __align__(8) uint64_t s_full[kNS], s_empty[kNS], s_recb[kRecs], s_based[kRecs];
+  wait_for_previous();
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 36) s_thr[threadIdx.x] = a.thr.thr[threadIdx.x];
@@ -682,8 +683,7 @@ static cudaError_t launch_c32(const CompressArgs& a, cudaStream_t st) {
   const uint32_t s_grid = (uint32_t)c;
   const uint32_t grid = a.ntiles < s_grid ? a.ntiles : s_grid;
   if (grid == 0) return cudaSuccess;
-  k<<<grid, kThreads, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_behind(k, grid, kThreads, smem, st, a);
 }
 
 cudaError_t launch_compress32(const CompressArgs& a, cudaStream_t st) { return launch_c32<false>(a, st); }
