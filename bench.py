@@ -278,7 +278,7 @@ def batched_workload(szp, torch, dev, T, nfields, reps=3, seed=11):
            "speedup": round(ms_single / ms_batch, 2),
            "tile_rounds": {"compress": cb.tile_rounds(), "decompress": db.tile_rounds()},
            "metric": "aggregate round-trip GB/s (compress + decompress, uncompressed bytes)",
-           "launches": "per field: 5 kernels x %d fields; batched: 2 graphs (5 kernels)" % nfields}
+           "launches": "per field: 4 kernels x %d fields; batched: 2 graphs (4 kernels)" % nfields}
     cb.close()
     db.close()
     return res
@@ -411,8 +411,7 @@ def config_leg(szp, torch, dev, T, x, eb, peak, reps=6):
     ABS bound eb, CUDA-event kernel times (first two round trips dropped).
     GB/s are uncompressed bytes (4n) per device time; each kernel's achieved
     bandwidth counts its algorithmic bytes (compress: 4n read + stream
-    written; locate: stream read + 4 B per block written; decode: stream and
-    block positions read + 4n written)."""
+    written; decode: stream read + 4n written)."""
     n = x.size
     dx = torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).to(dev)
     cap = szp.max_stream_bytes(n, L, T, 1)
@@ -432,13 +431,12 @@ def config_leg(szp, torch, dev, T, x, eb, peak, reps=6):
     torch.cuda.synchronize()
     assert szp.sync_status(st) == 0, szp.last_error()
     kt = {name: szp.kernel_time(slot) for slot, name in
-          enumerate(["rel_range", "compress", "dec_setup", "locate", "decode"])}
+          enumerate(["rel_range", "compress", "dec_setup", "locate", "decode"])}  # (locate: other blockSizes only)
     szp.set_timing(False)
     avg = {k: v[0] / v[1] for k, v in kt.items() if v[1]}
-    nb = 4.0 * n / L
-    alg = {"compress": 4.0 * n + size, "locate": size + nb, "decode": size + nb + 4.0 * n}
+    alg = {"compress": 4.0 * n + size, "decode": size + 4.0 * n}
     comp = avg["compress"]
-    dec = avg.get("dec_setup", 0) + avg["locate"] + avg["decode"]
+    dec = avg["dec_setup"] + avg["decode"]
     err = float((dx - dy).abs().max())
     return {"n": n, "abs_eb": eb, "stream_bytes": int(size), "ratio": round(4.0 * n / size, 3),
             "compress_gbs": round(4.0 * n / (comp / 1e3) / 1e9, 2),
@@ -638,8 +636,7 @@ def main():
     mean_out = float(np.mean([sizes[RELS[i % 3]] for i in range(args.steps)]))
     gbs = world * 4.0 * n * args.steps / (ms / 1e3) / 1e9
     # per-kernel achieved bandwidth from algorithmic bytes
-    alg = {"rel_range": 4.0 * n, "compress": 4.0 * n + mean_out, "dec_setup": 8.0 * T,
-           "locate": mean_out + 4.0 * n / L, "decode": mean_out + 4.0 * n + 4.0 * n / L}
+    alg = {"rel_range": 4.0 * n, "compress": 4.0 * n + mean_out, "dec_setup": 8.0 * T, "decode": mean_out + 4.0 * n}
     peak, peak_kind = measured_peak_gbs()
     kern = {}
     for k, (tot, cnt) in ktimes.items():
@@ -755,7 +752,7 @@ def main():
         del y1
         fm2 = {"rel": 1e-3, "ratio": round(4.0 * n / size2, 3),
                "compress_gbs": round(4.0 * n / ((avg["rel_range"] + avg["compress"]) / 1e3) / 1e9, 2),
-               "decompress_gbs": round(4.0 * n / ((avg["dec_setup"] + avg["locate"] + avg["decode"]) / 1e3) / 1e9, 2),
+               "decompress_gbs": round(4.0 * n / ((avg["dec_setup"] + avg["decode"]) / 1e3) / 1e9, 2),
                "kernels_ms": {k: round(v, 4) for k, v in avg.items()}}
         del d_s2
 
@@ -789,7 +786,7 @@ def main():
             assert errl <= ebl * (1 + 2.0 ** -22) + float(x.abs().max()) * 2.0 ** -22, \
                 "Lorenzo round trip exceeds the bound"
             c_ms = avg["rel_range"] + avg["codes"] + avg["compress"]
-            d_ms = avg["dec_setup"] + avg["locate"] + avg["decode"] + avg["inverse"]
+            d_ms = avg["dec_setup"] + avg["decode"] + avg["inverse"]
             lorenzo["by_rel"][str(rel)] = {
                 "ratio": round(4.0 * n / szl, 3), "fastmode1_ratio": round(4.0 * n / sizes[rel], 3),
                 "compress_gbs": round(4.0 * n / (c_ms / 1e3) / 1e9, 2),
@@ -824,8 +821,7 @@ def main():
         assert errd <= ebd * (1 + 1e-9), "float64 round trip exceeds the bound"
         f64 = {"n": nd, "rel": 1e-6, "ratio": round(8.0 * nd / szd, 3),
                "compress_gbs": round(8.0 * nd / ((avg["rel_range"] + avg["compress"]) / 1e3) / 1e9, 2),
-               "decompress_gbs": round(8.0 * nd / ((avg["dec_setup"] + avg["locate"] + avg["decode"]) / 1e3) / 1e9,
-                                       2),
+               "decompress_gbs": round(8.0 * nd / ((avg["dec_setup"] + avg["decode"]) / 1e3) / 1e9, 2),
                "kernels_ms": {k: round(v, 4) for k, v in avg.items()}}
         del xd, yd, d_sd
 
@@ -907,7 +903,7 @@ def main():
             "compress_gbs": round(world * 4.0 * n / (kern["compress"]["avg_ms"] / 1e3 +
                                                     kern.get("rel_range", {"avg_ms": 0})["avg_ms"] / 1e3) / 1e9, 2),
             "decompress_gbs": round(world * 4.0 * n / sum(kern[k]["avg_ms"] / 1e3 for k in
-                                                          ("dec_setup", "locate", "decode") if k in kern) / 1e9, 2),
+                                                          ("dec_setup", "decode") if k in kern) / 1e9, 2),
             "kernels": kern,
             "roofline": roof,
             "cpu_baseline": cpu,

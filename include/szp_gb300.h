@@ -313,7 +313,8 @@ int szp_gb300_wait_probe(unsigned long long limit_ns, unsigned long long *waited
 
 /* Per-kernel timing with CUDA events on the launching stream.  When enabled,
  * szp_gb300_kernel_ms(slot) returns the duration of the last launch of:
- * 0 REL range, 1 compress, 2 decompress setup, 3 locate, 4 decode, 5 the
+ * 0 REL range, 1 compress, 2 decompress setup, 3 locate (blockSizes other
+ * than 8..256 powers of two), 4 decode, 5 the
  * Lorenzo variant's codes pass, 6 its inverse sums (both of its passes). */
 void szp_gb300_set_timing(int enable);
 double szp_gb300_kernel_ms(int slot);
@@ -327,10 +328,8 @@ double szp_gb300_kernel_time(int slot, int *launches);
  * often and exercise the repair paths; streams decode the same. */
 void szp_gb300_set_locate_overlap(int bytes);
 
-/* Nonzero: a single field's decode pipeline draws tile tickets instead of its
- * cooperative launch with a static tile order (the path it takes when a
- * cooperative launch is refused, e.g. on a partitioned GPU); streams decode
- * the same.  0 restores the default. */
+/* Kept for callers that link it; changes nothing (the decoder always draws
+ * tickets, and needs no cooperative launch). */
 void szp_gb300_set_decode_tickets(int on);
 
 /* Chunks whose speculative header walk the last decompression of this
@@ -342,7 +341,7 @@ unsigned long long szp_gb300_kernel_launches(void);
 
 /* ---- batched fastmode1, blockSize 32 (no counterpart in the reference) ----
  * Many fields of uneven sizes and bounds go through one persistent launch per
- * stage (compress: range pass + tiles; decompress: header setup + locate +
+ * stage (compress: range pass + tiles; decompress: header setup +
  * decode), replayed as one CUDA graph.  Every field's stream is byte-identical
  * to szp_compress on that field alone with the same T.  All buffers are device
  * memory and must stay valid, and unchanged in size, for the batch's lifetime. */

@@ -503,8 +503,7 @@ def lorenzo_decompress_dev(d_stream, length, dims, d_out, segments=0, stream=0):
 
 
 def set_decode_tickets(on):
-    """Single-field decode with tile tickets instead of the cooperative static
-    schedule (the fallback path); for tests."""
+    """Kept for callers; changes nothing (the decoder always draws tickets)."""
     _lib.szp_gb300_set_decode_tickets(1 if on else 0)
 
 

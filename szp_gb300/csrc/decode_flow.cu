@@ -15,7 +15,7 @@
 //           predecessor did not leave where it entered walks again.
 //   sum     (fastmode1) all warps unpack the blocks' deltas once, for the sum of
 //           each group of 256 values
-//   look back  warp 0 publishes (block count, delta sum, entry, exit) and sums
+//   look back  the CTA publishes (block count, delta sum, entry, exit) and sums
 //           the predecessors' by a decoupled look-back over the segment, which
 //           also checks that the predecessor's exit is this entry; a wrong entry
 //           (rare) is corrected and walk and sum run again
@@ -29,8 +29,8 @@
 // bytes of index per block, a decode that held 32 KB of decoded values per tile
 // through a look-back over up to 304 tiles, two CTAs per SM) took 0.094 + 0.256
 // ms for a 512^3 field at REL 1e-3; here the bytes held are the compressed
-// ones, the stream is read once, and it takes 0.230 ms.  fastmode2, which has no
-// sum, went from 0.125 + 0.130 to 0.117 ms for 384^3 values in blocks of 64.
+// ones, the stream is read once, and it takes 0.225 ms.  fastmode2, which has no
+// sum, went from 0.125 + 0.130 to 0.120 ms for 384^3 values in blocks of 64.
 // Measured on the way, for the 512^3 field: a chain step with range checks took
 // 170 cycles, one without 70 (0.373 -> 0.316 ms with the branch-free walk); 8
 // CTAs of 64 registers spill, 0.26 ms; segments taken one after the other, not
@@ -332,7 +332,7 @@ __device__ __forceinline__ void shift_groups(uint32_t (&o)[2][8], const uint32_t
 // store_shifted for doubles, whose conversion is too long to have one copy of it
 // for each shift and each end: the ends go through `ends` (16 words of shared
 // memory), one element per lane.  (For floats the seven copies are the faster:
-// 232 us against 238 on a 168 Mvalue field.)
+// 232 us against 238 on 134 M values.)
 __device__ __forceinline__ void store_doubles(Put<kOutDouble>& put, unsigned long long* dst, const uint32_t (&q)[2][8], uint32_t V,
                                               int sh, int lane, uint32_t* ends) {
   __syncwarp();
@@ -870,7 +870,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       // Lane l of warp 0 reads the record at distance 1 + l; where none of those 32
       // is inclusive (a stream of one segment has all the CTAs in flight behind one
       // another) the four warps go on with 128 records a trip.  (Four windows from
-      // the start: 255 us instead of 232 on a 168 Mvalue field in 1024 segments.)
+      // the start: 255 us instead of 232 on 134 M values in 16 segments.)
       // A window that is not ready is read again; a broken chain of (entry, exit)
       // pairs (an older tile will correct itself) starts the look-back over.  A
       // tile whose entry is not its neighbour's exit walks again at once, from that
@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       // and publishes a second aggregate, so that the wrong entries of a segment
       // are mended side by side and not each after the prefixes of the one before
       // (2 M values of one segment whose entries are often wrong: 123 -> 85 us;
-      // the 168 Mvalue field 233 -> 225).  When that was not the true entry either,
+      // 134 M values in 16 segments 233 -> 225).  When that was not the true entry either,
       // the next walk waits until the whole chain is known.
       const int64_t first = (int64_t)rec - s_t.j;
       const uint32_t sc = s_t.sc;

@@ -22,8 +22,8 @@ __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Launches k behind the launch before it in the stream (with the decode's
-// status words cleared by its first kernel: a round trip of 20,000 values 64 ->
-// 55 us, a decode of 168 M values 240 -> 234); under stream capture in the
+// status words cleared by its first kernel: a round trip of 4,099 values 64 ->
+// 55 us, a decode of 134 M values 240 -> 234); under stream capture in the
 // ordinary way, so that the graph has plain edges only.
 template <typename... P>
 inline cudaError_t launch_behind(void (*k)(P...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t st,
