@@ -64,7 +64,7 @@ struct Shape {
   static constexpr uint32_t NB = 16384 / C;                        // chunks
   static constexpr uint32_t W = C / 2;                             // bytes walked before a chunk to find its entry
   static constexpr uint32_t LEAD2 = W < 4096 ? 4096 : W;           // bytes staged before a super-chunk, fastmode2
-  static constexpr uint32_t CAPL = 2048 / NB;                      // blocks a lane notes while it walks
+  static constexpr uint32_t CAPL = 2048 / NB;                      // blocks noted by a lane of a full super-chunk
   static constexpr uint32_t KCAP = LPB <= 4 ? 1536 : 512;          // blocks listed at a time
 };
 
@@ -405,9 +405,9 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
   extern __shared__ __align__(16) uint8_t s_b[];
   __shared__ uint16_t s_pos[KCAP];          // headers of the listed blocks (shared-memory offsets)
   __shared__ uint32_t s_tot[KCAP / BPR + 1];  // delta sums of the groups, then their exclusive prefixes
-  __shared__ uint16_t s_note[NB * CAPL + 32];  // the blocks that walking lanes note, CAPL for each chunk
-  constexpr uint32_t RUNS = 4;
-  __shared__ uint2 s_runs[NB][RUNS];  // and the runs of empty blocks they took at once: (notes before, first offset), length
+  __shared__ uint16_t s_note[NB * CAPL + 32];  // the blocks that walking lanes note
+  constexpr uint32_t RUNS = 128;
+  __shared__ uint2 s_runs[RUNS];  // and the runs of empty blocks they took at once: (notes before, first offset), length
   __shared__ uint32_t s_notes[NB];    // notes | runs << 16
   __shared__ uint32_t s_tried[kFlowWarps][32];
   __shared__ uint32_t s_ent[NB];            // entries of the chunks (shared-memory offsets, kDead: none found)
@@ -635,6 +635,11 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
     __syncthreads();
 
     // ---- walk: warp 0, a chunk per lane, from its entry ----
+    // the chunks share the room for notes (a super-chunk of mostly empty blocks has
+    // few chunks with many blocks each: 2^26 values of a walk at REL 1e-3, where
+    // 128 notes a chunk were too few, 300 -> 154 us; a mixed batch 530 -> 461; an
+    // 8192^2 field of runs pays for the run-time strides, 222 -> 231)
+    const uint32_t lg = 32 - __clz((lE - lS - 1) / C);  // 1 << lg chunks at least
     // region position of a shared-memory offset, kEnd past the region
     auto reg = [&](uint32_t p) -> uint32_t { return p - off >= rlen ? kEnd : p - off; };
     const uint32_t cS = lS + min((uint32_t)lane, NB) * C, cE = min(cS + C, lE);
@@ -759,7 +764,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           uint32_t p = go ? e + off : kAway, kk = 0;
           uint32_t nn = 0, nruns = 0;  // notes; runs of empty blocks
           const uint32_t chunk = min((uint32_t)lane, NB - 1);
-          uint16_t* const nt = s_note + chunk * CAPL;
+          uint16_t* const nt = s_note + chunk * (NB * CAPL >> lg);
           uint16_t* const spare = s_note + NB * CAPL + lane;  // a store here instead of a branch around one
           uint32_t over = kDead;  // how far past the chunk's end its chain crosses it
           do {
@@ -767,7 +772,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             pp[0] = p;
 #pragma unroll
             for (int u = 0; u < 4; u++) pp[u + 1] = ch.next(pp[u], b);
-            const bool room = nn + 4 <= CAPL;
+            const bool room = nn + 4 <= NB * CAPL >> lg;
             uint32_t n = 0;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -777,14 +782,14 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
               over = min(over, pp[u + 1] - cE);
             }
             kk += n;
-            nn += room ? n : n + CAPL;  // too many: nn > CAPL from here on
+            nn += room ? n : NB * CAPL;  // too many: past the limit from here on
             p = pp[4];
             if (p - pp[0] == 4 * Chain<LPB, FM2>::kEmpty && p < cE) {  // a run of empty blocks is taken at once
               const uint32_t first = p, k0 = kk;
               ch.zeros(p, cE, kk);
               over = min(over, p - cE);
               if (kk != k0) {
-                if (nruns < RUNS) s_runs[chunk][nruns] = make_uint2(nn << 16 | first, kk - k0);
+                if (nruns < RUNS >> lg) s_runs[chunk * (RUNS >> lg) + nruns] = make_uint2(nn << 16 | first, kk - k0);
                 nruns++;
               }
             }
@@ -792,7 +797,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           if (need) {
             k = kk;
             x = go ? (over > MAXSZ ? kDead : reg(cE + over)) : e;
-            noted = nn <= CAPL && nruns <= RUNS;
+            noted = nn <= NB * CAPL >> lg && nruns <= RUNS >> lg;
             s_notes[lane] = nn | nruns << 16;
           }
           // a lane's entry is its predecessor's exit; one that was not goes again
@@ -829,19 +834,21 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       }
       __syncthreads();
       if (s_noted) {  // gather the lanes' notes
-        constexpr uint32_t TPC = kFlowThreads / NB;  // threads per chunk
-        const uint32_t i = tid / TPC, c0 = s_c0[i], n = s_c0[i + 1] - c0;
+        const uint32_t i = tid * (1u << lg) / kFlowThreads, TPC = kFlowThreads >> lg;  // threads per chunk
+        const uint32_t c0 = s_c0[i], n = s_c0[i + 1] - c0;
+        const uint16_t* const nt = s_note + i * (NB * CAPL >> lg);
+        const uint2* const rn = s_runs + i * (RUNS >> lg);
         const uint32_t nn = n ? s_notes[i] & 0xFFFFu : 0u, nruns = n ? s_notes[i] >> 16 : 0u;
         if (nruns == 0) {
-          for (uint32_t t = tid % TPC; t < nn; t += TPC) s_pos[c0 + t] = s_note[i * CAPL + t];
+          for (uint32_t t = tid & (TPC - 1); t < nn; t += TPC) s_pos[c0 + t] = nt[t];
         } else {  // between its runs of empty blocks
           uint32_t t0 = 0, at = c0;
           for (uint32_t g = 0; g <= nruns; g++) {
-            const uint2 run = g < nruns ? s_runs[i][g] : make_uint2(nn << 16, 0);
+            const uint2 run = g < nruns ? rn[g] : make_uint2(nn << 16, 0);
             const uint32_t t1 = run.x >> 16;
-            for (uint32_t t = t0 + tid % TPC; t < t1; t += TPC) s_pos[at + t - t0] = s_note[i * CAPL + t];
+            for (uint32_t t = t0 + (tid & (TPC - 1)); t < t1; t += TPC) s_pos[at + t - t0] = nt[t];
             at += t1 - t0;
-            for (uint32_t t = tid % TPC; t < run.y; t += TPC) s_pos[at + t] = (uint16_t)((run.x & 0xFFFFu) + t * Chain<LPB, FM2>::kEmpty);
+            for (uint32_t t = tid & (TPC - 1); t < run.y; t += TPC) s_pos[at + t] = (uint16_t)((run.x & 0xFFFFu) + t * Chain<LPB, FM2>::kEmpty);
             at += run.y;
             t0 = t1;
           }

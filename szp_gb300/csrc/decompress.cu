@@ -92,21 +92,27 @@ __device__ void put_seed(const DecArgs& a, const DecField& fd, uint64_t e, uint3
   }
 }
 
-// Chunks in each super-chunk of a segment of nblk blocks in `bytes` bytes: as
-// many as hold 32 Ki values (empty blocks take one byte for 32 values, and a
-// CTA that meets thousands of them is the last to finish: a 2^24-value walk at
-// REL 1e-2 decodes 16 KB into 2 MB), and in a short stream no more than gives
-// the GPU one super-chunk per resident CTA (1 MB of floats: 22 -> 18 us), or
-// two of the same size where one each is not enough (21.5 MB in one segment as
-// 1312 super-chunks on 1064 CTAs: 208 us a call; as 1955: 162.  At three turns the
-// smaller ones lost 3 %).
+// Chunks in each super-chunk of a segment of nblk blocks in `bytes` bytes, of a
+// launch that decodes `values` values in `total` bytes and T segments in all:
+// - no more than hold 32 Ki values (empty blocks take one byte for 32 values, and
+//   a CTA that meets thousands of them is the last to finish: a 2^24-value walk
+//   at REL 1e-2 decodes 16 KB into 2 MB);
+// - where the resident CTAs (7 on each of 152 SMs) take one or two turns, as many
+//   as make these full and no third: 1 MB of floats 22 -> 18 us; 21.5 MB in one
+//   segment 208 -> 162 us a call (1312 super-chunks on 1064 CTAs became 1955);
+//   at three turns and more smaller super-chunks lost 3 %.
 __device__ __forceinline__ uint32_t flow_chunks(const DecArgs& a, uint64_t bytes, uint64_t nblk, uint32_t L,
-                                                uint64_t total) {
+                                                uint64_t total, uint64_t values, uint64_t T) {
   // in single precision: the result only has to be the same wherever it is taken
+  constexpr float kCtas = 1064.0f, kValues = 32768.0f;
   const float most = (float)(kFlowSuper / a.super_chunk), c = (float)a.super_chunk;
-  const float by_values = __fdiv_rn((float)bytes * (32768.0f / L), fmaxf((float)nblk, 1.0f) * c);
-  const float share = __fdiv_rn((float)total, 1024.0f * c), turns = ceilf(__fdiv_rn(share, most));
-  const float by_total = turns <= 1.0f ? share : turns <= 2.0f ? ceilf(__fdiv_rn(share, turns)) : most;
+  const float by_values = ceilf(__fdiv_rn((float)bytes * (kValues / L), fmaxf((float)nblk, 1.0f) * c));
+  const float turns = fmaxf(1.0f, ceilf(fmaxf(__fdiv_rn((float)total, kCtas * most * c),
+                                              __fdiv_rn((float)values, kCtas * kValues))));
+  // every segment may end in a short one
+  const float slots = fmaxf(kCtas * turns - (float)T, 0.5f * kCtas * turns);
+  const float by_total = turns <= 1.0f ? __fdiv_rn((float)total, 1024.0f * c)
+                         : turns <= 2.0f ? ceilf(__fdiv_rn((float)total, slots * c)) : most;
   return (uint32_t)fmaxf(1.0f, fminf(most, fminf(by_values, by_total)));
 }
 
@@ -151,7 +157,7 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   }
   // chunks per super-chunk, in its place in a ticket
   auto chunks = [&](uint64_t bytes, uint64_t nblk) -> uint32_t {
-    return flow_chunks(a, bytes, nblk, sg.L, gridDim.x * len) << kFlowFieldBits;
+    return flow_chunks(a, bytes, nblk, sg.L, gridDim.x * len, gridDim.x * sg.n, (uint64_t)gridDim.x * T) << kFlowFieldBits;
   };
   __syncthreads();
   for (uint32_t t = threadIdx.x; t < T; t += blockDim.x) {
@@ -216,14 +222,23 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   if (warp == 0) {  // chunk counts -> the chunks before each segment
     uint32_t acc = 0, most = 0;
     if (lane == 0) fd.chunk_base[0] = s_cb[0] = 0;
-    for (uint32_t t0 = 0; t0 < T; t0 += 32) {
-      const uint32_t t = t0 + lane;
-      const uint32_t n = t >= T || s_bad ? 0u : t < kTurnT ? s_cb[t + 1] : fd.chunk_base[t + 1];
-      const uint32_t incl = acc + warp_incl_scan(n, lane);
-      most = max(most, __reduce_max_sync(0xffffffffu, n));
-      if (t < T) fd.chunk_base[t + 1] = incl;
-      if (t < T && t < kTurnT) s_cb[t + 1] = incl;
-      acc = __shfl_sync(0xffffffffu, incl, 31);
+    for (uint32_t t0 = 0; t0 < T; t0 += 128) {  // four groups of loads in flight
+      uint32_t n[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const uint32_t t = t0 + 32 * u + lane;
+        n[u] = t >= T || s_bad ? 0u : t < kTurnT ? s_cb[t + 1] : fd.chunk_base[t + 1];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const uint32_t t = t0 + 32 * u + lane;
+        if (t0 + 32 * u >= T) break;
+        const uint32_t incl = acc + warp_incl_scan(n[u], lane);
+        most = max(most, __reduce_max_sync(0xffffffffu, n[u]));
+        if (t < T) fd.chunk_base[t + 1] = incl;
+        if (t < T && t < kTurnT) s_cb[t + 1] = incl;
+        acc = __shfl_sync(0xffffffffu, incl, 31);
+      }
     }
     if (lane == 0) {
       if (s_bad) atomicOr(fd.err, kErrCorrupt);
@@ -257,20 +272,28 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
       at += __popc(has);
     }
   }
-  // the rest, segment by segment; they come after the tickets of the turns
-  if (s_most <= turns) return;
-  uint32_t at = s_base0;
-  for (uint32_t t = 0; turns && t < T; t++) at += min(s_cb[t + 1] - s_cb[t], turns);
-  for (uint32_t t = 0; t < T; t++) {
-    const uint32_t c0 = t < kTurnT ? s_cb[t] : fd.chunk_base[t];
-    const uint32_t n = (t < kTurnT ? s_cb[t + 1] : fd.chunk_base[t + 1]) - c0;
-    if (n > turns) {
+  if (turns == 0) {  // segment by segment: the CTA each, or a thread each where there are many
+    const bool wide = T < 4;
+    for (uint32_t t = wide ? 0 : threadIdx.x; t < T; t += wide ? 1 : blockDim.x) {
+      const uint32_t c0 = t < kTurnT ? s_cb[t] : fd.chunk_base[t];
+      const uint32_t n = (t < kTurnT ? s_cb[t + 1] : fd.chunk_base[t + 1]) - c0;
+      if (n == 0) continue;
       const uint64_t len_t = sg.len(t);
       const uint32_t k = t < kTurnT ? s_k[t]
                                     : chunks(fd.reg1[t] - fd.reg0[t], a.fm2 ? (len_t + sg.L - 1) / sg.L : sg.blocks_fm1(t));
-      for (uint32_t j = turns + threadIdx.x; j < n; j += blockDim.x)
-        a.map[at + (j - turns)] = make_uint4(k | blockIdx.x, t, j, s_base0 + c0 + j);
+      for (uint32_t j = wide ? threadIdx.x : 0; j < n; j += wide ? blockDim.x : 1)
+        a.map[s_base0 + c0 + j] = make_uint4(k | blockIdx.x, t, j, s_base0 + c0 + j);
     }
+    return;
+  }
+  // the rest, segment by segment; they come after the tickets of the turns
+  if (s_most <= turns) return;
+  uint32_t at = s_base0;
+  for (uint32_t t = 0; t < T; t++) at += min(s_cb[t + 1] - s_cb[t], turns);
+  for (uint32_t t = 0; t < T; t++) {
+    const uint32_t c0 = s_cb[t], n = s_cb[t + 1] - c0;
+    for (uint32_t j = turns + threadIdx.x; j < n; j += blockDim.x)
+      a.map[at + (j - turns)] = make_uint4(s_k[t] | blockIdx.x, t, j, s_base0 + c0 + j);
     at += n > turns ? n - turns : 0u;
   }
 }
