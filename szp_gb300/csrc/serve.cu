@@ -274,6 +274,10 @@ int launch_group(szp_gb300_server_s& s, Lane& ln) {
     DecArgs a;
     args_decompress(a, dp, reinterpret_cast<DecField*>(tb_d + o_df), static_cast<uint4*>(ln.map.p), ln.misc->counters,
                     static_cast<uint64_t*>(ln.status.p), &ln.misc->ls, &ln.misc->err);
+    // lanes run side by side: with 7 of the decoder's small CTAs on every SM, another
+    // lane's compressor (two large CTAs per SM) finds no room until all of them
+    // have ended.  At 400k requests/s: 7 per SM 925-996 GB/s, 4 per SM 976-1031.
+    a.nlocate_ctas = std::min<uint32_t>(a.nlocate_ctas, 4u * (uint32_t)s.sms);
     rc = issue_decompress(a, (uint32_t)nd, ln.st);
     if (rc) return rc;
   }
