@@ -487,6 +487,9 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
             xv[0] = A.w; xv[1] = B.x; xv[2] = B.y; xv[3] = B.z; xv[4] = B.w; xv[5] = C.x; xv[6] = C.y; xv[7] = C.z;
           }
         }
+        // no eighth delta: what stands there is the next block's seed, or past the
+        // tile's last block a word that no copy wrote and no quantization may see
+        if (lone) xv[7] = xv[6];
       } else {
 #pragma unroll
         for (int j = 0; j < 8; j++) xv[j] = (uint32_t)j < ml ? sx[i + j] : 0.0f;
@@ -522,7 +525,6 @@ __global__ void __launch_bounds__(kPipeThreads, 2) compress_pipe(const __grid_co
       bseed[r] = prev;
       uint32_t sb = 0, lmax = 0;
       if (full) {
-        if (lone) q[7] = q[6];  // no eighth delta
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           const int32_t d = (int32_t)((uint32_t)q[j] - (uint32_t)prev);  // wrapping, as the compiled reference
