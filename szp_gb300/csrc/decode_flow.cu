@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         t.rlen = (uint32_t)(R1 - R0);
         t.sc = (at.x >> kFlowFieldBits) * C;
         t.scS = at.z * t.sc;
-        t.scE = min(t.scS + t.sc, t.rlen);
+        t.scE = t.scS + min(t.sc, t.rlen - t.scS);  // (a region may end a byte below 4 GiB)
         t.last = t.scE == t.rlen;
         const uint32_t lead = min(FM2 ? S::LEAD2 : S::W, a.overlap);
         t.st0 = t.scS > lead ? t.scS - lead : 0u;
@@ -919,7 +919,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           const int jstar = bi ? __ffs(bi) - 1 : 32;     // nearest inclusive of the window
           const bool rel = inr && lane <= jstar;
           const uint64_t vx = status_value(w.x), vy = status_value(w.y);
-          const uint32_t tS = (uint32_t)(idx - first) * sc, tE = min(tS + sc, rlen);
+          const uint32_t tS = (uint32_t)(idx - first) * sc, tE = tS + min(sc, rlen - tS);
           const uint32_t xr = (uint32_t)(vx & 1023u) | (uint32_t)(vy & 1023u) << 10;
           const uint32_t tx = xr == kXDead ? kDead : xr == kXEnd ? kEnd : tE + xr;
           const uint32_t hr = (uint32_t)(vx >> 26) & 0xFFFFu;
@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           uint32_t d[8], run = 0, seed = 0, bc = 0;
           if (FM2) {
             if (valid) {
-              if (o + 4 - off > rlen) {
+              if (rlen - (o - off) < 4) {
                 corrupt = true;
               } else {
                 seed = lds_le32(s_b, o);
@@ -1110,7 +1110,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           }
           if (m) {
             bc = o - off < rlen ? s_b[o] : 255u;
-            if (bc > 33 || o - off + block_bytes(m, bc) > rlen) {
+            if (bc > 33 || block_bytes(m, bc) > rlen - (o - off)) {
               corrupt = true;
               bc = 0;
             }

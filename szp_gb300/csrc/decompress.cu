@@ -331,12 +331,14 @@ struct SmemChain {
   bool fm2;
   // block size at p, 0 when its bit-count byte is invalid or not staged
   __device__ __forceinline__ uint32_t step(uint32_t p) const {
-    uint32_t hp = fm2 ? p + 4 : p;
-    if (hp >= avail) return 0;
-    const uint32_t b = sb[hp - base0];
+    const uint32_t skip = fm2 ? 4u : 0u;
+    if (p >= avail || avail - p <= skip) return 0;
+    const uint32_t b = sb[p + skip - base0];
     if (l8) return b > (uint32_t)kMaxBitCount ? 0u : (b ? 1 + l8 * (b + 1) : 1u);
     return full_block_size(b, L, fm2);
   }
+  // the position sz bytes on; past 2^32 (a region may end a byte below it) the last one there is
+  static __device__ __forceinline__ uint32_t after(uint32_t p, uint32_t sz) { return p + min(sz, 0xFFFFFFFFu - p); }
   // walk from p to cE: header count, exit (kPosEnd past the region, kPosDead)
   __device__ __forceinline__ uint32_t walk(uint32_t p, uint32_t cE, uint32_t* exit) const {
     uint32_t k = 0;
@@ -347,7 +349,7 @@ struct SmemChain {
         return k;
       }
       k++;
-      p += sz;
+      p = after(p, sz);
     }
     *exit = p >= rlen ? kPosEnd : p;
     return k;
@@ -368,7 +370,7 @@ __device__ __forceinline__ void rewalk_from(const SmemChain& ch, uint32_t* h, ui
       continue;
     }
     if (h[i] != e) {
-      const uint32_t cE = min(scS + (i + 1) * C, scE);
+      const uint32_t cE = scS + min((i + 1) * C, scE - scS);
       h[i] = e;
       uint32_t ex;
       k[i] = ch.walk(e, cE, &ex);
@@ -422,7 +424,7 @@ __global__ void __launch_bounds__(kLocThreads) locate_kernel(const __grid_consta
   const uint64_t R0 = fd.reg0[t];
   const uint32_t rlen = (uint32_t)(fd.reg1[t] - R0);
   const uint32_t C = a.chunk, SC = a.super_chunk, W0 = a.overlap;
-  const uint32_t scS = j * SC, scE = min(scS + SC, rlen);
+  const uint32_t scS = j * SC, scE = scS + min(SC, rlen - scS);
 
   // ---- stage [scS - W0, scE + maxsz) of the region ----
   const uint32_t st0 = scS > W0 ? scS - W0 : 0u;
@@ -470,7 +472,7 @@ __global__ void __launch_bounds__(kLocThreads) locate_kernel(const __grid_consta
   // times, but an iteration is a handful of instructions (a lockstep loop that
   // applied every outcome with selects cost several times as much).
   const uint32_t nactive = (scE - scS + C - 1) / C;
-  const uint32_t cS = scS + tid * C, cE = min(cS + C, scE);
+  const uint32_t cS = scS + tid * C, cE = (uint32_t)tid < nactive ? cS + min(C, scE - cS) : scE;
   uint32_t h = kPosEnd, x = kPosEnd, k = 0;
   if ((uint32_t)tid < nactive) {
     const bool known = j == 0 && tid == 0;  // a segment's block region starts with a header
@@ -492,7 +494,7 @@ __global__ void __launch_bounds__(kLocThreads) locate_kernel(const __grid_consta
       const uint32_t sz = b32 ? (b > (uint32_t)kMaxBitCount ? 0u : (b ? 4 * b + 5 : 1u)) : ch.step(pos);
       if (sz) {
         cnt += pos >= cS ? 1u : 0u;
-        const uint32_t np = pos + sz;
+        const uint32_t np = SmemChain::after(pos, sz);
         if (entry == kPosDead && np >= cS) entry = np;
         pos = np;
       } else if (!known && anchor + 1 < cE) {
@@ -586,7 +588,7 @@ __global__ void __launch_bounds__(kLocThreads) locate_kernel(const __grid_consta
               ready = status_epoch(s1) == (epoch & 0xFFFFF) && (f == kFlagAggregate || f == kFlagInclusive);
               incl = ready && f == kFlagInclusive;
               const uint64_t v = status_value(s1);
-              const uint32_t sS = (uint32_t)(idx - (int64_t)first) * SC, sE = min(sS + SC, rlen);
+              const uint32_t sS = (uint32_t)(idx - (int64_t)first) * SC, sE = sS + min(SC, rlen - sS);
               const uint32_t xr = (uint32_t)v & 0xFFu;
               ax.y = xr == kXDead ? kPosDead : xr == kXEnd ? kPosEnd : sE + xr;
               if (incl) {
