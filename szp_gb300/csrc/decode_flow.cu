@@ -8,7 +8,7 @@
 //           shared memory, where it stays until its values are written
 //   walk    the block headers are found.  The stream keeps no index: a block's
 //           position depends on every bit count before it in its segment.  The
-//           super-chunk is cut into 16 chunks; the warps first find where the
+//           super-chunk is cut into 1 to 16 chunks; the warps first find where the
 //           header chain crosses each chunk's start (chains started on payload
 //           die, a header byte must be <= 33, or fall in with the true chain), then
 //           a lane walks each chunk and notes its blocks.  A lane whose
@@ -32,7 +32,7 @@
 // ones, the stream is read once, and it takes 0.225 ms.  fastmode2, which has no
 // sum, went from 0.125 + 0.130 to 0.120 ms for 384^3 values in blocks of 64.
 // Measured on the way, for the 512^3 field: a chain step with range checks took
-// 170 cycles, one without 70 (0.373 -> 0.316 ms with the branch-free walk); 8
+// 170 cycles, one without 55 (0.373 -> 0.316 ms with the branch-free walk); 8
 // CTAs of 64 registers spill, 0.26 ms; segments taken one after the other, not
 // in turns, 0.373 against 0.291 ms.
 #include <atomic>
@@ -54,19 +54,38 @@ constexpr int kFlowThreads = 32 * kFlowWarps;
 constexpr uint32_t kEnd = 0xFFFFFFFEu;   // the walk left the segment region
 constexpr uint32_t kDead = 0xFFFFFFFFu;  // the walk met an invalid header
 
-// Shape of the decoder for blocks of 8*LPB values: about 16 KB of stream per
-// CTA, cut into chunks of at least 7 blocks of the largest size.
+// Shape of the decoder for blocks of 8*LPB values: up to 16 KB of stream per
+// CTA, cut into 2 to 16 chunks that hold 7 blocks of the largest size.
 template <int LPB>
 struct Shape {
   static constexpr uint32_t L = 8 * LPB;
-  static constexpr uint32_t BPR = 32 / LPB;                        // blocks per group of 256 values
-  static constexpr uint32_t C = LPB <= 4 ? 1024 : 256 * LPB;       // bytes per chunk (a walking lane)
-  static constexpr uint32_t NB = 16384 / C;                        // chunks
-  static constexpr uint32_t W = C / 2;                             // bytes walked before a chunk to find its entry
-  static constexpr uint32_t LEAD2 = W < 4096 ? 4096 : W;           // bytes staged before a super-chunk, fastmode2
-  static constexpr uint32_t CAPL = 2048 / NB;                      // blocks noted by a lane of a full super-chunk
-  static constexpr uint32_t KCAP = LPB <= 4 ? 1536 : 512;          // blocks listed at a time
+  static constexpr uint32_t BPR = 32 / LPB;                   // blocks per group of 256 values
+  static constexpr uint32_t C = LPB <= 4 ? 1024 : 256 * LPB;  // bytes per chunk (a walking lane)
+  static constexpr uint32_t CL = LPB <= 4 ? 10 : LPB == 8 ? 11 : LPB == 16 ? 12 : 13;
+  static constexpr uint32_t NB = kFlowSuper / C;              // chunks
+  static constexpr uint32_t KCAP = LPB <= 4 ? 1536 : LPB == 8 ? 1024 : LPB == 16 ? 768 : 512;  // blocks listed at a time
+  static_assert(C == 1u << CL, "chunks of a power of two");
 };
+
+// fastmode1 blocks of 8 and 16 values may take little more than a byte each, and
+// a lane's walk is a chain of dependent steps: the setup kernel gives them
+// chunks of down to C / 8 (flow_shape).  (33.5 M values in blocks of 8 at 0.23
+// bytes a value: 1.62 ms with chunks of C, 0.24 so.  For blocks of 32 the
+// run-time chunk cost 3 % at ordinary bounds.)
+template <int LPB, bool FM2>
+constexpr bool kVarChunks = LPB <= 2 && !FM2;
+// Bytes walked before a chunk to find its entry: 4 or more of the largest blocks,
+// and half of it before shorter chunks of 16-value blocks (always half: more
+// wrong entries, 33.5 M values in one segment at 1.33 bytes a value 115 -> 176 us;
+// never: 134 M values at 0.09 bytes a value 441 -> 597 us).
+template <int LPB>
+constexpr uint32_t kWindow = LPB == 1 ? 128 : Shape<LPB>::C / 2;
+template <int LPB, bool FM2>
+constexpr uint32_t kLead = FM2 ? 4096 : kWindow<LPB>;  // bytes staged before a super-chunk
+// Runs of empty blocks that the walking lanes note (134 M values in blocks of 8 at
+// 0.18 bytes a value, where 128 are too few: 719 -> 660 us).
+template <int LPB, bool FM2>
+constexpr uint32_t kRuns = kVarChunks<LPB, FM2> ? 256 : 128;
 
 template <int LPB, bool FM2>
 __host__ __device__ constexpr uint32_t flow_maxsz() {
@@ -79,7 +98,7 @@ __host__ __device__ constexpr uint32_t flow_maxsz() {
 // phase, the last block's rest, and what loads read past a block's end.
 template <int LPB, bool FM2>
 __host__ __device__ constexpr uint32_t flow_smem() {
-  return 16 + (FM2 ? Shape<LPB>::LEAD2 : Shape<LPB>::W) + Shape<LPB>::C * Shape<LPB>::NB + flow_maxsz<LPB, FM2>() + 8 + 32;
+  return 16 + kLead<LPB, FM2> + kFlowSuper + flow_maxsz<LPB, FM2>() + 8 + 32;
 }
 
 // The super-chunk a CTA is working on.
@@ -93,6 +112,7 @@ struct FlowTile {
   uint32_t tile, j, rec, last;  // ticket; position in the segment; look-back record; whether it is the last
   uint32_t strict;          // another segment follows: the region holds the segment's blocks and no more
   uint32_t sc;              // bytes of the segment's super-chunks
+  uint32_t cl;              // log2 of their chunks' bytes
   uint32_t scS, scE, rlen;  // region offsets of the super-chunk and the region's length
   uint32_t st0, st1;        // region offsets of the staged bytes
   uint32_t align;           // shared-memory offset of the first staged byte
@@ -401,13 +421,14 @@ template <int LPB, bool BATCH, bool FM2, int OUT>
 __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_constant__ DecArgs a) {
   using S = Shape<LPB>;
   constexpr uint32_t L = S::L, BPR = S::BPR, KCAP = S::KCAP, MAXSZ = flow_maxsz<LPB, FM2>();
-  constexpr uint32_t C = S::C, NB = S::NB, CAPL = S::CAPL;
+  constexpr uint32_t NB = S::NB, WIN = kWindow<LPB>, NOTES = kFlowNotes, RUNS = kRuns<LPB, FM2>;
   extern __shared__ __align__(16) uint8_t s_b[];
   __shared__ uint16_t s_pos[KCAP];          // headers of the listed blocks (shared-memory offsets)
   __shared__ uint32_t s_tot[KCAP / BPR + 1];  // delta sums of the groups, then their exclusive prefixes
-  __shared__ uint16_t s_note[NB * CAPL + 32];  // the blocks that walking lanes note
-  constexpr uint32_t RUNS = 128;
-  __shared__ uint2 s_runs[RUNS];  // and the runs of empty blocks they took at once: (notes before, first offset), length
+  __shared__ uint16_t s_note[NOTES + 32];  // the blocks that walking lanes note
+  // and the runs of empty blocks they took at once: notes before << 16 | first offset; length
+  __shared__ uint32_t s_runs[RUNS];
+  __shared__ uint16_t s_len[RUNS];
   __shared__ uint32_t s_notes[NB];    // notes | runs << 16
   __shared__ uint32_t s_tried[kFlowWarps][32];
   __shared__ uint32_t s_ent[NB];            // entries of the chunks (shared-memory offsets, kDead: none found)
@@ -436,21 +457,23 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       const uint32_t tile = draw_ticket_persistent(a.ls, total);
       s_t.tile = tile;
       if (tile < total) {
-        const uint4 at = a.map[tile];  // field and chunks, segment, position in it, look-back record
-        const DecField& fd = BATCH ? a.fields[at.x & kFlowFieldMask] : a.f;
+        const uint4 at = a.map[tile];  // field, segment, position in it and shape, look-back record
+        const DecField& fd = BATCH ? a.fields[at.x] : a.f;
         const Segments sg = fd.seg;
         const uint64_t R0 = fd.reg0[at.y], R1 = fd.reg1[at.y];
         FlowTile t;
         t.tile = tile;
-        t.j = at.z;
+        t.j = at.z & kFlowPosMask;
         t.rec = at.w;
         t.strict = at.y + 1 < sg.T;
         t.rlen = (uint32_t)(R1 - R0);
-        t.sc = (at.x >> kFlowFieldBits) * C;
-        t.scS = at.z * t.sc;
+        const uint32_t shape = at.z >> kFlowPosBits;
+        t.cl = S::CL - (kVarChunks<LPB, FM2> ? shape >> 4 : 0u);
+        t.sc = ((shape & 15) + 1) << t.cl;
+        t.scS = t.j * t.sc;
         t.scE = t.scS + min(t.sc, t.rlen - t.scS);  // (a region may end a byte below 4 GiB)
         t.last = t.scE == t.rlen;
-        const uint32_t lead = min(FM2 ? S::LEAD2 : S::W, a.overlap);
+        const uint32_t lead = min(kLead<LPB, FM2>, a.overlap);
         t.st0 = t.scS > lead ? t.scS - lead : 0u;
         t.st1 = (uint32_t)min((uint64_t)t.rlen, (uint64_t)t.scE + MAXSZ + 8);
         // the 16-byte-aligned part of the staged bytes that lies in the stream goes by bulk copy
@@ -481,7 +504,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         t.eb = fd.plan->eb;
         t.ebd = fd.plan->ebd;
         t.seed = 0;
-        if (!FM2 && at.z == 0) {
+        if (!FM2 && t.j == 0) {
           const uint8_t* sp = fd.in + R0 - 4;  // the segment's 4-byte seed precedes its blocks
           t.seed = (uint32_t)__ldg(sp) | ((uint32_t)__ldg(sp + 1) << 8) | ((uint32_t)__ldg(sp + 2) << 16) |
                    ((uint32_t)__ldg(sp + 3) << 24);
@@ -506,9 +529,10 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
     const Chain<LPB, FM2> ch{s_b, s_t.st1 + off, flow_smem<LPB, FM2>() - 8};
     const uint32_t scS = s_t.scS, scE = s_t.scE, rlen = s_t.rlen;
     const bool j0 = s_t.j == 0;
+    const uint32_t cl = kVarChunks<LPB, FM2> ? s_t.cl : S::CL;  // log2 of a chunk's bytes
 
     // ---- entries: where the header chain crosses each chunk's start ----
-    // 32 lanes walk from 32 neighbouring bytes W before the chunk.  Chains that
+    // 32 lanes walk from 32 neighbouring bytes, WIN or less before the chunk.  Chains that
     // began on payload meet an invalid header or fall in with the true one; the
     // position that most of them reach is taken (a wrong one is corrected below;
     // 2 in 1000 are, of a walk at REL 1e-3).  Where all die (blocks longer than 32
@@ -522,10 +546,10 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       uint32_t open = 0;     // chunks without an entry yet
 #pragma unroll
       for (int q = 0; q < Q; q++) {
-        const uint32_t i = warp + kFlowWarps * q, B = lS + i * C;
+        const uint32_t i = warp + kFlowWarps * q, B = lS + (i << cl);
         const uint32_t first = s_t.st0 + off;
-        back[q] = S::W;
-        at[q] = B - first > S::W ? B - S::W : first;
+        back[q] = WIN >> (kVarChunks<LPB, FM2> && LPB == 2 && cl < S::CL);
+        at[q] = B - first > back[q] ? B - back[q] : first;
         p[q] = kAway;
         if (i < NB && B < lE && !(i == 0 && j0)) {
           open |= 1u << q;
@@ -541,7 +565,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
 #pragma unroll
         for (int q = 0; q < Q; q++) {
           if (!(open >> q & 1)) continue;
-          const uint32_t B = lS + (warp + kFlowWarps * q) * C, g = (B & ~15u) - 512 + 16 * lane;
+          const uint32_t B = lS + ((warp + kFlowWarps * q) << cl), g = (B & ~15u) - 512 + 16 * lane;
           const bool in = (int32_t)g >= (int32_t)at[q];
           const uint4 v = in ? *reinterpret_cast<const uint4*>(s_b + g) : make_uint4(1, 0, 0, 0);
           uint32_t m = __ballot_sync(0xffffffffu, (v.x | v.y | v.z | v.w) == 0);
@@ -559,27 +583,27 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         // three steps from 32 bytes of each chunk; most chains that began on payload die here
         uint32_t b, past[Q];  // past: how far past the chunk's start its chain crosses it
 #pragma unroll
-        for (int q = 0; q < Q; q++) past[q] = p[q] - (lS + (warp + kFlowWarps * q) * C);
+        for (int q = 0; q < Q; q++) past[q] = p[q] - (lS + ((warp + kFlowWarps * q) << cl));
 #pragma unroll
         for (int u = 0; u < 3; u++)
 #pragma unroll
           for (int q = 0; q < Q; q++) {
             p[q] = ch.next(p[q], b);
-            past[q] = min(past[q], p[q] - (lS + (warp + kFlowWarps * q) * C));  // the first past it: the smallest
+            past[q] = min(past[q], p[q] - (lS + ((warp + kFlowWarps * q) << cl)));  // the first past it: the smallest
           }
         __syncwarp();
         if (lane < 8 * Q) tried[lane] = kAway;
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-          const uint32_t B = lS + (warp + kFlowWarps * q) * C;
+          const uint32_t B = lS + ((warp + kFlowWarps * q) << cl);
           const bool alive = (p[q] < kAway || past[q] <= MAXSZ) && at[q] + lane < B;
           const uint32_t m = __ballot_sync(0xffffffffu, alive), n = __popc(m & ((1u << lane) - 1u));
           if (alive && n < 8) tried[8 * q + n] = past[q] <= MAXSZ ? B + past[q] : p[q];
         }
         __syncwarp();
         // lanes 8q .. 8q + 7: the first 8 survivors of chunk q, on to its start
-        const uint32_t B = lS + (warp + kFlowWarps * min((uint32_t)lane >> 3, (uint32_t)Q - 1)) * C;
+        const uint32_t B = lS + ((warp + kFlowWarps * min((uint32_t)lane >> 3, (uint32_t)Q - 1)) << cl);
         uint32_t c = lane < 8 * Q ? tried[lane] : kAway, over = c - B;
         bool busy = c < B;
         while (__any_sync(0xffffffffu, busy)) {
@@ -615,7 +639,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           p[q] = kAway;
           if (!(open >> q & 1)) continue;
           if (FM2 && (split >> (8 * q) & 0xFFu)) {
-            const uint32_t first = s_t.st0 + off, Bq = lS + (warp + kFlowWarps * q) * C;
+            const uint32_t first = s_t.st0 + off, Bq = lS + ((warp + kFlowWarps * q) << cl);
             if (Bq - first > back[q]) {
               back[q] *= 4;
               at[q] = Bq - first > back[q] ? Bq - back[q] : first;
@@ -624,7 +648,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             }
           }
           at[q] += 32;
-          if ((found >> (8 * q) & 1) || at[q] >= lS + (warp + kFlowWarps * q) * C) {
+          if ((found >> (8 * q) & 1) || at[q] >= lS + ((warp + kFlowWarps * q) << cl)) {
             open &= ~(1u << q);
           } else {
             p[q] = at[q] + lane;
@@ -639,10 +663,10 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
     // few chunks with many blocks each: 2^26 values of a walk at REL 1e-3, where
     // 128 notes a chunk were too few, 300 -> 154 us; a mixed batch 530 -> 461; an
     // 8192^2 field of runs pays for the run-time strides, 222 -> 231)
-    const uint32_t lg = 32 - __clz((lE - lS - 1) / C);  // 1 << lg chunks at least
+    const uint32_t lg = 32 - __clz((lE - lS - 1) >> cl);  // 1 << lg chunks at least
     // region position of a shared-memory offset, kEnd past the region
     auto reg = [&](uint32_t p) -> uint32_t { return p - off >= rlen ? kEnd : p - off; };
-    const uint32_t cS = lS + min((uint32_t)lane, NB) * C, cE = min(cS + C, lE);
+    const uint32_t cS = lS + (min((uint32_t)lane, NB) << cl), cE = min(cS + (1u << cl), lE);
     const bool act = warp == 0 && lane < (int)NB && cS < cE;
     // the super-chunk's entry (region position); a segment's block region starts with a header
     uint32_t h0 = 0, e0 = kDead;
@@ -764,15 +788,15 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           uint32_t p = go ? e + off : kAway, kk = 0;
           uint32_t nn = 0, nruns = 0;  // notes; runs of empty blocks
           const uint32_t chunk = min((uint32_t)lane, NB - 1);
-          uint16_t* const nt = s_note + chunk * (NB * CAPL >> lg);
-          uint16_t* const spare = s_note + NB * CAPL + lane;  // a store here instead of a branch around one
+          uint16_t* const nt = s_note + chunk * (NOTES >> lg);
+          uint16_t* const spare = s_note + NOTES + lane;  // a store here instead of a branch around one
           uint32_t over = kDead;  // how far past the chunk's end its chain crosses it
           do {
             uint32_t pp[5], b;
             pp[0] = p;
 #pragma unroll
             for (int u = 0; u < 4; u++) pp[u + 1] = ch.next(pp[u], b);
-            const bool room = nn + 4 <= NB * CAPL >> lg;
+            const bool room = nn + 4 <= NOTES >> lg;
             uint32_t n = 0;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -782,14 +806,17 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
               over = min(over, pp[u + 1] - cE);
             }
             kk += n;
-            nn += room ? n : NB * CAPL;  // too many: past the limit from here on
+            nn += room ? n : NOTES;  // too many: past the limit from here on
             p = pp[4];
             if (p - pp[0] == 4 * Chain<LPB, FM2>::kEmpty && p < cE) {  // a run of empty blocks is taken at once
               const uint32_t first = p, k0 = kk;
               ch.zeros(p, cE, kk);
               over = min(over, p - cE);
               if (kk != k0) {
-                if (nruns < RUNS >> lg) s_runs[chunk * (RUNS >> lg) + nruns] = make_uint2(nn << 16 | first, kk - k0);
+                if (nruns < RUNS >> lg) {
+                  s_runs[chunk * (RUNS >> lg) + nruns] = nn << 16 | first;
+                  s_len[chunk * (RUNS >> lg) + nruns] = (uint16_t)(kk - k0);
+                }
                 nruns++;
               }
             }
@@ -797,7 +824,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           if (need) {
             k = kk;
             x = go ? (over > MAXSZ ? kDead : reg(cE + over)) : e;
-            noted = nn <= NB * CAPL >> lg && nruns <= RUNS >> lg;
+            noted = nn <= NOTES >> lg && nruns <= RUNS >> lg;
             s_notes[lane] = nn | nruns << 16;
           }
           // a lane's entry is its predecessor's exit; one that was not goes again
@@ -836,20 +863,20 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       if (s_noted) {  // gather the lanes' notes
         const uint32_t i = tid * (1u << lg) / kFlowThreads, TPC = kFlowThreads >> lg;  // threads per chunk
         const uint32_t c0 = s_c0[i], n = s_c0[i + 1] - c0;
-        const uint16_t* const nt = s_note + i * (NB * CAPL >> lg);
-        const uint2* const rn = s_runs + i * (RUNS >> lg);
+        const uint16_t* const nt = s_note + i * (NOTES >> lg);
+        const uint32_t r0 = i * (RUNS >> lg);
         const uint32_t nn = n ? s_notes[i] & 0xFFFFu : 0u, nruns = n ? s_notes[i] >> 16 : 0u;
         if (nruns == 0) {
           for (uint32_t t = tid & (TPC - 1); t < nn; t += TPC) s_pos[c0 + t] = nt[t];
         } else {  // between its runs of empty blocks
           uint32_t t0 = 0, at = c0;
           for (uint32_t g = 0; g <= nruns; g++) {
-            const uint2 run = g < nruns ? rn[g] : make_uint2(nn << 16, 0);
-            const uint32_t t1 = run.x >> 16;
+            const uint32_t run = g < nruns ? s_runs[r0 + g] : nn << 16, len = g < nruns ? s_len[r0 + g] : 0u;
+            const uint32_t t1 = run >> 16;
             for (uint32_t t = t0 + (tid & (TPC - 1)); t < t1; t += TPC) s_pos[at + t - t0] = nt[t];
             at += t1 - t0;
-            for (uint32_t t = tid & (TPC - 1); t < run.y; t += TPC) s_pos[at + t] = (uint16_t)((run.x & 0xFFFFu) + t * Chain<LPB, FM2>::kEmpty);
-            at += run.y;
+            for (uint32_t t = tid & (TPC - 1); t < len; t += TPC) s_pos[at + t] = (uint16_t)((run & 0xFFFFu) + t * Chain<LPB, FM2>::kEmpty);
+            at += len;
             t0 = t1;
           }
         }

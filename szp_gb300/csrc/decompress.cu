@@ -92,28 +92,43 @@ __device__ void put_seed(const DecArgs& a, const DecField& fd, uint64_t e, uint3
   }
 }
 
-// Chunks in each super-chunk of a segment of nblk blocks in `bytes` bytes, of a
-// launch that decodes `values` values in `total` bytes and T segments in all:
+// Shape (szp_kernels.h) of the super-chunks of a segment of nblk blocks in
+// `bytes` bytes, of a launch that decodes `values` values in `total` bytes and T
+// segments in all (a batch takes its fields to be like this one):
 // - no more than hold 32 Ki values (empty blocks take one byte for 32 values, and
 //   a CTA that meets thousands of them is the last to finish: a 2^24-value walk
-//   at REL 1e-2 decodes 16 KB into 2 MB);
-// - where the resident CTAs (7 on each of 152 SMs) take one or two turns, as many
-//   as make these full and no third: 1 MB of floats 22 -> 18 us; 21.5 MB in one
-//   segment 208 -> 162 us a call (1312 super-chunks on 1064 CTAs became 1955);
-//   at three turns and more smaller super-chunks lost 3 %.
-__device__ __forceinline__ uint32_t flow_chunks(const DecArgs& a, uint64_t bytes, uint64_t nblk, uint32_t L,
-                                                uint64_t total, uint64_t values, uint64_t T) {
+//   at REL 1e-2 decodes 16 KB into 2 MB) or about 1024 blocks (the list of
+//   them has 1536 places; 33.5 M values in blocks of 8 at 0.48 bytes a value: 299
+//   -> 207 us);
+// - where 1064 CTAs (7 on each of 152 SMs; the server runs fewer) take one or two
+//   turns, as many as make these full and no third: 1 MB of floats 22 -> 18 us;
+//   21.5 MB in one segment 208 -> 162 us a call (1312 super-chunks on 1064 CTAs
+//   became 1955); at three turns and more smaller super-chunks lost 3 %;
+// - fastmode1 blocks of 8 and 16 values: of shorter chunks, as far as that needs no more
+//   than 16 of them (decode_flow.cu, kVarChunks);
+// - no more chunks than leave each the room to note 5/4 of its blocks (134 M values in
+//   blocks of 32 at 0.26 bytes a value: 412 -> 317 us).
+__device__ __forceinline__ uint32_t flow_shape(const DecArgs& a, uint64_t bytes, uint64_t nblk, uint32_t L,
+                                               uint64_t total, uint64_t values, uint64_t T) {
   // in single precision: the result only has to be the same wherever it is taken
-  constexpr float kCtas = 1064.0f, kValues = 32768.0f;
+  constexpr float kCtas = 1064.0f;
+  const float blocks = fminf(32768.0f / (float)L, 1024.0f), most_values = blocks * (float)L;
   const float most = (float)(kFlowSuper / a.super_chunk), c = (float)a.super_chunk;
-  const float by_values = ceilf(__fdiv_rn((float)bytes * (kValues / L), fmaxf((float)nblk, 1.0f) * c));
+  const float fit = __fdiv_rn((float)bytes * blocks, fmaxf((float)nblk, 1.0f) * c);  // chunks that hold `blocks`
   const float turns = fmaxf(1.0f, ceilf(fmaxf(__fdiv_rn((float)total, kCtas * most * c),
-                                              __fdiv_rn((float)values, kCtas * kValues))));
+                                              __fdiv_rn((float)values, kCtas * most_values))));
   // every segment may end in a short one
   const float slots = fmaxf(kCtas * turns - (float)T, 0.5f * kCtas * turns);
   const float by_total = turns <= 1.0f ? __fdiv_rn((float)total, 1024.0f * c)
                          : turns <= 2.0f ? ceilf(__fdiv_rn((float)total, slots * c)) : most;
-  return (uint32_t)fmaxf(1.0f, fminf(most, fminf(by_values, by_total)));
+  const uint32_t s = L <= 16 && !a.fm2 ? (fit <= 2.0f ? 3 : fit <= 4.0f ? 2 : fit <= 8.0f ? 1 : 0) : 0;
+  const float u = (float)(1u << s);
+  // whole chunks, but not above 1300 blocks
+  const float by_blocks = s ? ceilf(fit * u) : fminf(ceilf(fit), floorf(fit * 1.27f));
+  const float share = (float)kFlowNotes * 0.8f * fit * u / blocks;  // chunks whose blocks have room
+  const float by_notes = share >= 16.0f ? 16.0f : share >= 8.0f ? 8.0f : share >= 4.0f ? 4.0f : share >= 2.0f ? 2.0f : 1.0f;
+  const float k = fminf(fminf(by_notes, most * u), fminf(by_blocks, floorf(by_total * u)));
+  return s << 4 | ((uint32_t)fmaxf(u, k) - 1);
 }
 
 template <bool BATCH>
@@ -124,7 +139,7 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   const uint32_t hb = a.hb == 8 ? 8u : 4u;  // eb header: float, or double (szpd_double.cc)
   const uint64_t head = hb + 8ull * T;
   constexpr uint32_t kTurnT = 512;  // segments at most for the turns below
-  __shared__ uint32_t s_cb[kTurnT + 1], s_k[kTurnT];  // tickets before each segment; its chunks per super-chunk
+  __shared__ uint32_t s_cb[kTurnT + 1], s_k[kTurnT];  // tickets before each segment; its shape
   __shared__ uint32_t s_bad, s_base0, s_all, s_most;  // s_most: of the segment with the most super-chunks
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   if (!BATCH) {
@@ -155,9 +170,9 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
     fd.plan->eb = eb;
     fd.plan->ebd = ebd;
   }
-  // chunks per super-chunk, in its place in a ticket
-  auto chunks = [&](uint64_t bytes, uint64_t nblk) -> uint32_t {
-    return flow_chunks(a, bytes, nblk, sg.L, gridDim.x * len, gridDim.x * sg.n, (uint64_t)gridDim.x * T) << kFlowFieldBits;
+  // a segment's shape, in its place in a ticket
+  auto shape_of = [&](uint64_t bytes, uint64_t nblk) -> uint32_t {
+    return flow_shape(a, bytes, nblk, sg.L, gridDim.x * len, gridDim.x * sg.n, (uint64_t)gridDim.x * T) << kFlowPosBits;
   };
   __syncthreads();
   for (uint32_t t = threadIdx.x; t < T; t += blockDim.x) {
@@ -197,8 +212,9 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
             if (r1 - r0 >= (1ull << 32)) bad = true;  // block offsets are 32-bit
             uint32_t sc = a.super_chunk;
             if (a.map) {
-              k = chunks(r1 - r0, nblk);
-              sc *= k >> kFlowFieldBits;
+              k = shape_of(r1 - r0, nblk);
+              const uint32_t shape = k >> kFlowPosBits;
+              sc = ((shape & 15) + 1) * (sc >> (shape >> 4));
             }
             nch = (uint32_t)((r1 - r0 + sc - 1) / sc);
           }
@@ -268,7 +284,7 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
       const uint32_t c0 = s_cb[min(t, T)], n = t < T ? s_cb[t + 1] - c0 : 0u;
       const uint32_t has = __ballot_sync(0xffffffffu, n > j);
       if (n > j)
-        a.map[at + __popc(has & ((1u << lane) - 1u))] = make_uint4(s_k[t] | blockIdx.x, t, j, s_base0 + c0 + j);
+        a.map[at + __popc(has & ((1u << lane) - 1u))] = make_uint4(blockIdx.x, t, s_k[t] | j, s_base0 + c0 + j);
       at += __popc(has);
     }
   }
@@ -280,9 +296,9 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
       if (n == 0) continue;
       const uint64_t len_t = sg.len(t);
       const uint32_t k = t < kTurnT ? s_k[t]
-                                    : chunks(fd.reg1[t] - fd.reg0[t], a.fm2 ? (len_t + sg.L - 1) / sg.L : sg.blocks_fm1(t));
+                                    : shape_of(fd.reg1[t] - fd.reg0[t], a.fm2 ? (len_t + sg.L - 1) / sg.L : sg.blocks_fm1(t));
       for (uint32_t j = wide ? threadIdx.x : 0; j < n; j += wide ? blockDim.x : 1)
-        a.map[s_base0 + c0 + j] = make_uint4(k | blockIdx.x, t, j, s_base0 + c0 + j);
+        a.map[s_base0 + c0 + j] = make_uint4(blockIdx.x, t, k | j, s_base0 + c0 + j);
     }
     return;
   }
@@ -293,7 +309,7 @@ __global__ void dec_setup_kernel(const __grid_constant__ DecArgs a) {
   for (uint32_t t = 0; t < T; t++) {
     const uint32_t c0 = s_cb[t], n = s_cb[t + 1] - c0;
     for (uint32_t j = turns + threadIdx.x; j < n; j += blockDim.x)
-      a.map[at + (j - turns)] = make_uint4(s_k[t] | blockIdx.x, t, j, s_base0 + c0 + j);
+      a.map[at + (j - turns)] = make_uint4(blockIdx.x, t, s_k[t] | j, s_base0 + c0 + j);
     at += n > turns ? n - turns : 0u;
   }
 }

@@ -147,8 +147,14 @@ struct DecArgs {
 };
 
 // Stream bytes of a decode_flow super-chunk at most, and the bits of a ticket's
-// field number (its chunks stand above them).
-constexpr uint32_t kFlowSuper = 16384, kFlowFieldBits = 26, kFlowFieldMask = (1u << kFlowFieldBits) - 1;
+// position in its segment (a region is below 4 GiB and a super-chunk takes 1 KB).
+// Above them stands the shape of the segment's super-chunks: their chunks - 1
+// (4 bits), and by how many bits the chunks are shorter than flow_chunk_bytes.
+constexpr uint32_t kFlowSuper = 16384, kFlowPosBits = 22, kFlowPosMask = (1u << kFlowPosBits) - 1;
+// Blocks of a super-chunk that its walking lanes note, an equal share for each chunk
+// (of a power of two of them); where there is no room, warp 0 lists the blocks
+// in a second walk.
+constexpr uint32_t kFlowNotes = 2048;
 
 // What decode_flow writes: floats, doubles (float64 streams), the int32 codes,
 // or the codes added to those already there (the homomorphic reduction).
@@ -199,7 +205,7 @@ cudaError_t launch_decode_f64(const DecArgs& a, cudaStream_t st);
 cudaError_t launch_dec_setup_batch(const DecArgs& a, uint32_t nfields, cudaStream_t st);
 // blockSize 8..256, a power of two (decode_flow.cu); a batch is fastmode1, blockSize 32
 bool flow_supported(uint32_t L);
-uint32_t flow_chunk_bytes(uint32_t L);  // a super-chunk is 1 to 16 KB / this many of them
+uint32_t flow_chunk_bytes(uint32_t L);  // of a chunk at most; a super-chunk takes this much to 16 KB
 cudaError_t launch_decode_flow(const DecArgs& a, cudaStream_t st);
 cudaError_t launch_decode_flow_batch(const DecArgs& a, cudaStream_t st);
 cudaError_t prepare_decompress_batch();
