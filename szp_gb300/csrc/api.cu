@@ -1436,7 +1436,7 @@ int szp_gb300_lorenzo_decompress_dev(const unsigned char* d_bytes, size_t byteLe
     cudaError_t e = launch_lorenzo_inverse(a, (uint32_t)w->sm_count, st);
     w->mark(kSlotLorenzoInv, 1, st);
     if (e != cudaSuccess) rc = fail(SZP_GB300_ECUDA, "Lorenzo inverse passes: %s", cudaGetErrorString(e));
-    count_launches(2);
+    count_launches(nz > 1 ? 2 : 1);
   }
   if (rc == SZP_GB300_OK) rc = finish_sync(*w, st, nullptr);
   w->end(st);
