@@ -201,8 +201,9 @@ struct Packer {
   }
 };
 
-// Launches one group on a lane.
-int launch_group(szp_gb300_server_s& s, Lane& ln) {
+// Launches one group on a lane; `behind`: other lanes run beside it, and more
+// requests wait than the lanes take in two turns.
+int launch_group(szp_gb300_server_s& s, Lane& ln, bool behind) {
   const int L = (int)kBatchL, T = s.T;
   std::vector<szp_gb300_field> cf, df;
   ln.cidx.assign(ln.reqs.size(), -1);
@@ -274,10 +275,14 @@ int launch_group(szp_gb300_server_s& s, Lane& ln) {
     DecArgs a;
     args_decompress(a, dp, reinterpret_cast<DecField*>(tb_d + o_df), static_cast<uint4*>(ln.map.p), ln.misc->counters,
                     static_cast<uint64_t*>(ln.status.p), &ln.misc->ls, &ln.misc->err);
-    // lanes run side by side: with 7 of the decoder's small CTAs on every SM, another
-    // lane's compressor (two large CTAs per SM) finds no room until all of them
-    // have ended.  At 400k requests/s: 7 per SM 925-996 GB/s, 4 per SM 976-1031.
-    a.nlocate_ctas = std::min<uint32_t>(a.nlocate_ctas, 4u * (uint32_t)s.sms);
+    // With 7 of the decoder's small CTAs on every SM another lane's compressor (two
+    // large CTAs per SM) finds no room until all of them have ended: a server that
+    // is behind gives them 2, and one that keeps up ends the group sooner with 7.
+    // 20 runs of 20,000 requests each, median GB/s and p99: at 400k requests/s 2 per SM
+    // 1070, 15.6 ms, 4 per SM 1022, 18.7, 7 per SM 962, 22.6; at 200k requests/s the p50 is
+    // 0.334 ms with 2, 0.293 with 4, 0.282 with 7.
+    const uint32_t per_sm = behind ? 2u : 7u;
+    a.nlocate_ctas = std::min<uint32_t>(a.nlocate_ctas, per_sm * (uint32_t)s.sms);
     rc = issue_decompress(a, (uint32_t)nd, ln.st);
     if (rc) return rc;
   }
@@ -359,8 +364,9 @@ void worker_main(szp_gb300_server_s* s) {
       free_lane->reqs = group;
       free_lane->busy = true;
       s->in_flight++;
+      const bool behind = s->lanes.size() > 1 && s->queue.size() > 2 * (size_t)s->cfg.max_batch * s->lanes.size();
       lk.unlock();
-      int rc = launch_group(*s, *free_lane);
+      int rc = launch_group(*s, *free_lane, behind);
       lk.lock();
       if (rc) {
         s->worker_status = rc;
