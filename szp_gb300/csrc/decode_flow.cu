@@ -783,7 +783,8 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       if (warp == 0) {
         uint32_t e = lane == 0 ? h0 : e0, k = 0, x = kDead;
         bool need = act, noted = true;
-        while (__any_sync(0xffffffffu, need)) {
+        uint32_t differ;
+        do {
           const bool go = need && e != kDead && e != kEnd && e + off < cE;
           uint32_t p = go ? e + off : kAway, kk = 0;
           uint32_t nn = 0, nruns = 0;  // notes; runs of empty blocks
@@ -827,13 +828,27 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
             noted = nn <= NOTES >> lg && nruns <= RUNS >> lg;
             s_notes[lane] = nn | nruns << 16;
           }
-          // a lane's entry is its predecessor's exit; one that was not goes again
+          // A lane's entry is its predecessor's exit; one that was not goes again.  Of
+          // neighbours that were not only the first goes (the others' predecessors are
+          // to change), and none goes by a walk that died: that is most often one to
+          // be mended itself, and the lanes behind it, which had been right, went the
+          // same way one after the other, each a walk (4 us) of its own: 64 us in one of
+          // the 1060 super-chunks of a segment, which the next 800 waited for.
           const uint32_t px = __shfl_up_sync(0xffffffffu, x, 1);
-          need = lane > 0 && act && px != e;
+          differ = __ballot_sync(0xffffffffu, lane > 0 && act && px != e && px != kDead);
+          need = (differ & ~(differ << 1)) >> lane & 1;
           if (need) {
             e = px;
             repaired = true;
           }
+        } while (differ);
+        // behind a walk that died on the chain itself there are no blocks
+        const uint32_t dead = __ballot_sync(0xffffffffu, act && x == kDead);
+        if (dead && act && lane >= __ffs(dead)) {
+          e = x = kDead;
+          k = 0;
+          noted = true;
+          s_notes[lane] = 0;
         }
         // exit, count and each lane's first block
         const uint32_t nact = __popc(__ballot_sync(0xffffffffu, act));

@@ -112,7 +112,7 @@ __device__ __forceinline__ uint32_t flow_shape(const DecArgs& a, uint64_t bytes,
                                                uint64_t total, uint64_t values, uint64_t T) {
   // in single precision: the result only has to be the same wherever it is taken
   constexpr float kCtas = 1064.0f;
-  const float blocks = fminf(32768.0f / (float)L, 1024.0f), most_values = blocks * (float)L;
+  const float blocks = (float)min(32768u >> (31 - __clz(L)), 1024u), most_values = blocks * (float)L;  // L: a power of two
   const float most = (float)(kFlowSuper / a.super_chunk), c = (float)a.super_chunk;
   const float fit = __fdiv_rn((float)bytes * blocks, fmaxf((float)nblk, 1.0f) * c);  // chunks that hold `blocks`
   const float turns = fmaxf(1.0f, ceilf(fmaxf(__fdiv_rn((float)total, kCtas * most * c),
@@ -125,8 +125,9 @@ __device__ __forceinline__ uint32_t flow_shape(const DecArgs& a, uint64_t bytes,
   const float u = (float)(1u << s);
   // whole chunks, but not above 1300 blocks
   const float by_blocks = s ? ceilf(fit * u) : fminf(ceilf(fit), floorf(fit * 1.27f));
-  const float share = (float)kFlowNotes * 0.8f * fit * u / blocks;  // chunks whose blocks have room
-  const float by_notes = share >= 16.0f ? 16.0f : share >= 8.0f ? 8.0f : share >= 4.0f ? 4.0f : share >= 2.0f ? 2.0f : 1.0f;
+  const float room = (float)kFlowNotes * 0.8f * fit * u;  // `blocks` times the chunks whose blocks have room
+  const float by_notes = room >= 16.0f * blocks ? 16.0f : room >= 8.0f * blocks ? 8.0f : room >= 4.0f * blocks ? 4.0f
+                         : room >= 2.0f * blocks ? 2.0f : 1.0f;
   const float k = fminf(fminf(by_notes, most * u), fminf(by_blocks, floorf(by_total * u)));
   return s << 4 | ((uint32_t)fmaxf(u, k) - 1);
 }
