@@ -417,6 +417,31 @@ __device__ __forceinline__ void store_groups(Put<OUT>& put, E* dst, const uint32
   }
 }
 
+// Lists blocks [kb, kb + cap) of a super-chunk whose blocks are more than the list
+// holds, from what the walking lanes noted of its 1 << lg chunks: the blocks between
+// a chunk's runs of empty ones (E bytes each), and the runs.  All threads.
+// Out of line: few super-chunks come here, and inlined it cost every other 3 %.
+static __device__ __noinline__ void gather_window(uint16_t* pos, const uint16_t* note, const uint32_t* notes,
+                                                  const uint32_t* runs, const uint16_t* lens, const uint32_t* c0s,
+                                                  uint32_t note_share, uint32_t run_share, uint32_t lg, uint32_t kb,
+                                                  uint32_t cap, uint32_t E) {
+  const uint32_t tid = threadIdx.x, TPC = kFlowThreads >> lg, i = tid / TPC, first = tid & (TPC - 1);  // threads per chunk
+  const uint32_t c0 = c0s[i], n = c0s[i + 1] - c0;
+  const uint32_t nn = n ? notes[i] & 0xFFFFu : 0u, nruns = n ? notes[i] >> 16 : 0u;
+  uint32_t t0 = 0, at = c0 - kb;  // the next note, and its place in the list (before the list: wraps around)
+  for (uint32_t g = 0; g <= nruns; g++) {
+    const uint32_t run = g < nruns ? runs[i * run_share + g] : nn << 16, len = g < nruns ? lens[i * run_share + g] : 0u;
+    const uint32_t t1 = run >> 16;
+    for (uint32_t t = t0 + first; t < t1; t += TPC)
+      if (at + t - t0 < cap) pos[at + t - t0] = note[i * note_share + t];
+    at += t1 - t0;
+    for (uint32_t t = first; t < len; t += TPC)
+      if (at + t < cap) pos[at + t] = (uint16_t)((run & 0xFFFFu) + t * E);
+    at += len;
+    t0 = t1;
+  }
+}
+
 template <int LPB, bool BATCH, bool FM2, int OUT>
 __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_constant__ DecArgs a) {
   using S = Shape<LPB>;
@@ -433,7 +458,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
   __shared__ uint32_t s_tried[kFlowWarps][32];
   __shared__ uint32_t s_ent[NB];            // entries of the chunks (shared-memory offsets, kDead: none found)
   __shared__ uint32_t s_c0[NB + 1];         // blocks before each chunk
-  __shared__ bool s_noted;                  // the walking lanes noted every block
+  __shared__ bool s_noted, s_many;          // the walking lanes noted every block and run; and there are more than KCAP
   __shared__ FlowTile s_t;
   __shared__ uint32_t s_k, s_sum, s_h0, s_epoch;
   __shared__ FlowWindow s_win[kFlowWarps];
@@ -855,7 +880,8 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         xl = __shfl_sync(0xffffffffu, x, nact - 1);
         const uint32_t incl = warp_incl_scan(k, lane);
         K = __shfl_sync(0xffffffffu, incl, 31);
-        noted = __all_sync(0xffffffffu, noted) && K <= KCAP;
+        const bool all_noted = __all_sync(0xffffffffu, noted);
+        noted = all_noted && K <= KCAP;
         wi0 = incl - k;
         wn = incl;
         wp0 = e + off;  // e is a position where k > 0
@@ -871,8 +897,9 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           s_k = K;
           s_h0 = h0;
           s_noted = noted;
+          s_many = all_noted && K > KCAP;
         }
-        if (!noted) list(0);
+        if (!all_noted) list(0);
       }
       __syncthreads();
       if (s_noted) {  // gather the lanes' notes
@@ -900,9 +927,13 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       K = s_k;
       sum = 0;
       for (uint32_t kb = 0; kb < K && !FM2; kb += KCAP) {
-        if (kb) {
+        if (kb || s_many) {
           __syncthreads();
-          if (warp == 0) list(kb);
+          if (s_many) {
+            gather_window(s_pos, s_note, s_notes, s_runs, s_len, s_c0, NOTES >> lg, RUNS >> lg, lg, kb, KCAP, Chain<LPB, FM2>::kEmpty);
+          } else if (warp == 0) {
+            list(kb);
+          }
           __syncthreads();
         }
         sum += sums(min(KCAP, K - kb));
@@ -1060,7 +1091,9 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       const uint32_t kn = min(KCAP, kmax - kb);
       if (K > KCAP) {  // more blocks than the list holds: list them again
         __syncthreads();
-        if (warp == 0) {
+        if (s_many) {
+          gather_window(s_pos, s_note, s_notes, s_runs, s_len, s_c0, NOTES >> lg, RUNS >> lg, lg, kb, KCAP, Chain<LPB, FM2>::kEmpty);
+        } else if (warp == 0) {
           if (kb == 0) {
             wi = wi0;
             wp = wp0;
