@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
         } while (differ);
         // behind a walk that died on the chain itself there are no blocks
         const uint32_t dead = __ballot_sync(0xffffffffu, act && x == kDead);
-        if (dead && act && lane >= __ffs(dead)) {
+        if (__builtin_expect(dead && act && lane >= __ffs(dead), false)) {
           e = x = kDead;
           k = 0;
           noted = true;
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
           s_noted = noted;
           s_many = all_noted && K > KCAP;
         }
-        if (!all_noted) list(0);
+        if (__builtin_expect(!all_noted, false)) list(0);
       }
       __syncthreads();
       if (s_noted) {  // gather the lanes' notes
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
       K = s_k;
       sum = 0;
       for (uint32_t kb = 0; kb < K && !FM2; kb += KCAP) {
-        if (kb || s_many) {
+        if (__builtin_expect(kb || s_many, false)) {
           __syncthreads();
           if (s_many) {
             gather_window(s_pos, s_note, s_notes, s_runs, s_len, s_c0, NOTES >> lg, RUNS >> lg, lg, kb, KCAP, Chain<LPB, FM2>::kEmpty);
@@ -1089,7 +1089,7 @@ __global__ void __launch_bounds__(kFlowThreads, 7) decode_flow(const __grid_cons
     bool corrupt = false;
     for (uint32_t kb = 0; kb < kmax; kb += KCAP) {
       const uint32_t kn = min(KCAP, kmax - kb);
-      if (K > KCAP) {  // more blocks than the list holds: list them again
+      if (__builtin_expect(K > KCAP, false)) {  // more blocks than the list holds: list them again
         __syncthreads();
         if (s_many) {
           gather_window(s_pos, s_note, s_notes, s_runs, s_len, s_c0, NOTES >> lg, RUNS >> lg, lg, kb, KCAP, Chain<LPB, FM2>::kEmpty);
