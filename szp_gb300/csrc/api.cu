@@ -895,11 +895,6 @@ void host_tile_counts(size_t n, int T, int L, uint32_t tb, uint64_t& tiles_per_s
   Segments sg = make_segments(n, T, L);
   tile_counts(sg, false, tb, tiles_per_seg, ntiles);
 }
-uint64_t host_block_count(size_t n, int T, int L) {
-  Segments sg = make_segments(n, T, L);
-  if (!sg.n) return 0;
-  return (uint64_t)(sg.T - 1) * (sg.tsz ? seg_blocks_host(sg, 0, false) : 0) + seg_blocks_host(sg, sg.T - 1, false);
-}
 size_t host_max_stream_bytes(size_t n, int L, int T) { return max_stream_bytes(n, L, T, 1); }
 int host_status_from_err(uint32_t err) { return status_from_err(err); }
 void host_segment_blocks(size_t n, int T, int L, uint64_t& nb_reg, uint64_t& nb_last) {

@@ -1,7 +1,7 @@
 // decode_flow.cu -- the fastmode1 / fastmode2 decoder for blockSize 8..256 (a
 // power of two): one kernel from stream bytes to values.
 //
-// A segment's stream is cut into super-chunks of about 16 KB and each CTA takes
+// A segment's stream is cut into super-chunks of 1 to 16 KB and each CTA takes
 // one at a time, in ticket order:
 //
 //   stage   one bulk copy brings the super-chunk (and a lead-in before it) to
@@ -23,14 +23,15 @@
 //           scans them in registers, dequantizes and stores them, 32 bytes per
 //           lane, with no further exchange between warps
 //
-// What bounds it: the logic pipe (half of the SM's issue rate) and, with 7 CTAs
-// of 4 warps per SM, the waits between the steps of a super-chunk; not HBM.
+// What bounds it: the waits between the steps of a super-chunk.  With 7 CTAs of 4
+// warps per SM, issue is 65 % and the ALU 56 % busy, DRAM 30 %; the largest stall is
+// the barrier, where three warps wait while one walks (2^26 values at REL 1e-3).
 // Why this shape: the pipeline it replaces (a pass that located blocks, 4
 // bytes of index per block, a decode that held 32 KB of decoded values per tile
 // through a look-back over up to 304 tiles, two CTAs per SM) took 0.094 + 0.256
 // ms for a 512^3 field at REL 1e-3; here the bytes held are the compressed
-// ones, the stream is read once, and it takes 0.225 ms.  fastmode2, which has no
-// sum, went from 0.125 + 0.130 to 0.120 ms for 384^3 values in blocks of 64.
+// ones, the stream is read once, and it takes 0.208 ms.  fastmode2, which has no
+// sum, went from 0.125 + 0.130 to 0.104 ms for 384^3 values in blocks of 64.
 // Measured on the way, for the 512^3 field: a chain step with range checks took
 // 170 cycles, one without 55 (0.373 -> 0.316 ms with the branch-free walk); 8
 // CTAs of 64 registers spill, 0.26 ms; segments taken one after the other, not

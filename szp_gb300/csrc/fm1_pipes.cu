@@ -159,12 +159,10 @@ __device__ __forceinline__ void c32_producer(const CompressArgs& a, uint8_t* slo
 // (the eb header for the first tile, the decoupled look-back for the others),
 // the segment offset of a segment's first tile and the stream size after the
 // last tile.  The position goes back to the compute warps in the record.
-template <bool QI>
 __device__ __forceinline__ void c32_control(const CompressArgs& a, const C32Meta* meta, C32Rec* rec, uint64_t* recb,
                                             uint64_t* based, const uint32_t* s_epoch,
                                             const volatile uint32_t* s_stop_k, float eb) {
   const int lane = threadIdx.x & 31;
-  const uint32_t hb = QI ? a.qhb : 4;  // bytes of the eb header: float64 streams carry a double
   for (uint32_t k = 0;; k++) {
     const int p = (int)(k % kRecs);
     if (!control_wait_full(&recb[p], (k / kRecs) & 1, k, s_stop_k, a.err)) return;
@@ -174,20 +172,16 @@ __device__ __forceinline__ void c32_control(const CompressArgs& a, const C32Meta
     const uint32_t epoch = *s_epoch;
     uint64_t excl = 0;
     if (m.tile == 0) {
-      if (QI && hb == 8) {
-        write_header_warp(a.out, a.ebd_dev ? *a.ebd_dev : a.ebd, a.seg, lane);
-      } else {
-        write_header_warp(a.out, eb, a.seg, lane);
-      }
+      write_header_warp(a.out, eb, a.seg, lane);
     } else {
       excl = lookback_sum(a.status, m.tile, 0, epoch, a.err);
       if (lane == 0) st_relaxed_u64(a.status + m.tile, make_status(epoch, kFlagInclusive, excl + agg));
     }
     if (lane == 0) {
-      const uint64_t gpos = hb + 8ull * a.seg.T + excl;
+      const uint64_t gpos = 4 + 8ull * a.seg.T + excl;
       const bool fits = gpos + agg <= a.cap;
       if (m.tile == a.ntiles - 1) *a.out_size = gpos + agg;
-      if (m.first && fits) write_offset(a.out, m.seg, excl, hb);
+      if (m.first && fits) write_offset(a.out, m.seg, excl);
       if (!fits) atomicOr(a.err, kErrCapacity);
       r.dst = fits ? a.out + gpos : nullptr;
       mbar_arrive(&based[p]);
@@ -428,8 +422,8 @@ __device__ __forceinline__ void c32_pack_masked(uint8_t* dst, const uint32_t (&v
   }
 }
 
-// QI: the input is int32 codes (float64 data quantized by a pass before, or the
-// homomorphic sum's).
+// QI: the input is int32 codes under a float header (the homomorphic sum's, the
+// Lorenzo variant's).
 template <bool QI>
 __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_constant__ CompressArgs a) {
   extern __shared__ __align__(16) uint8_t s_dyn[];
@@ -468,7 +462,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress32_pipe(const __grid_cons
     return;
   }
   if (warp == kW) {
-    c32_control<QI>(a, s_meta, s_rec, s_recb, s_based, &s_epoch, &s_cstop_k, eb);
+    c32_control(a, s_meta, s_rec, s_recb, s_based, &s_epoch, &s_cstop_k, eb);
     return;
   }
 

@@ -230,7 +230,6 @@ void host_compress_tiles(size_t n, int T, int L, uint64_t& tiles_per_seg, uint64
                          uint32_t& bpw);
 void host_segment_blocks(size_t n, int T, int L, uint64_t& nb_reg, uint64_t& nb_last);
 void host_tile_counts(size_t n, int T, int L, uint32_t tb, uint64_t& tiles_per_seg, uint64_t& ntiles);
-uint64_t host_block_count(size_t n, int T, int L);
 size_t host_max_stream_bytes(size_t n, int L, int T);
 int host_status_from_err(uint32_t err);
 int host_fail(int status, const char* msg);
