@@ -71,7 +71,7 @@ struct Shape {
 // fastmode1 blocks of 8 and 16 values may take little more than a byte each, and
 // a lane's walk is a chain of dependent steps: the setup kernel gives them
 // chunks of down to C / 8 (flow_shape).  (33.5 M values in blocks of 8 at 0.23
-// bytes a value: 1.62 ms with chunks of C, 0.24 so.  For blocks of 32 the
+// bytes a value: 0.46 ms with chunks of C, 0.16 so.  For blocks of 32 the
 // run-time chunk cost 3 % at ordinary bounds.)
 template <int LPB, bool FM2>
 constexpr bool kVarChunks = LPB <= 2 && !FM2;
